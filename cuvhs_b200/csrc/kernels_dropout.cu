@@ -7,9 +7,9 @@
 // over those classes is a "last decisive class" scan, so each segment's
 // incoming state comes from one prefix pass instead of the reference's
 // one-thread-per-field walk.  The short list of state changes is then merged,
-// filtered and mapped to TBC lines in order by one thread, and one warp
-// conceals the entries column step by column step (all loads of a step before
-// its stores), which is how the reference's copy loop behaves.
+// filtered and mapped to TBC lines in order by prefix sums, and the entries
+// are concealed a thread per column, each pixel from where the reference's
+// copy loop (column step by column step) would have taken it.
 //
 // Two forms share those steps:
 //  * two-pass (the decoder): a wide class kernel (one thread per block, every
@@ -30,17 +30,18 @@ namespace cuvhs {
 namespace {
 
 constexpr int kThreadsD = 256;       // fused kernel and class kernel
-constexpr int kThreadsScan = 512;    // two-pass scan kernel
+constexpr int kThreadsScan = 1024;   // two-pass scan kernel: a thread per column of an NTSC line
 constexpr int kMaxEvents = 2048;
 constexpr int kStage = kThreadsD * 16;  // envelope samples one class CTA stages
 constexpr int kMaxEnvBlocks = 1024;     // envelope partials a class CTA holds in shared memory
 
-__device__ int find_line(const double* ll, int als, int n, double pos) {
-  if (pos < ll[als] || pos >= ll[als + n]) return -1;
+// Index of the line holding pos among the n lines whose starts are ll[0..n].
+__device__ int find_line(const double* ll, int n, double pos) {
+  if (pos < ll[0] || pos >= ll[n]) return -1;
   int lo = 0, hi = n - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) / 2;
-    if (ll[als + mid] <= pos) lo = mid;
+    if (ll[mid] <= pos) lo = mid;
     else hi = mid - 1;
   }
   return lo;
@@ -66,80 +67,204 @@ __device__ __forceinline__ unsigned char block_class(double sum, int n, double d
   return m <= down ? 0 : (m >= up ? 1 : 2);  // 0 = at/below down, 1 = at/above up, 2 = between
 }
 
-// Step 4 (thread 0): merge start/end events (<= 30 samples apart), keep <= 128
-// spans, drop spans < 10 samples, map to TBC lines.  Returns the entry count.
-__device__ int map_events(const DropoutArgs& a, int f, const int* events, int ne, int s0, int s1, int* rf_s,
-                          int* rf_e) {
-  const double* ll = a.ll + (size_t)f * a.lines_per_frame;
-  const int als = a.active_line_start, H = a.out_h, W = a.out_w;
+// Block-wide exclusive sum over THREADS threads (warp shuffles, then the warp
+// totals).  wsh holds 32 ints; every thread must call.
+template <int THREADS>
+__device__ __forceinline__ int block_excl_sum(int v, int* wsh, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NW = THREADS / 32;
+  int x = v;
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, x, off);
+    if (lane >= off) x += o;
+  }
+  if (lane == 31) wsh[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    int w = lane < NW ? wsh[lane] : 0;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, w, off);
+      if (lane >= off) w += o;
+    }
+    if (lane < NW) wsh[lane] = w;  // inclusive warp prefix
+  }
+  __syncthreads();
+  const int res = x - v + (warp > 0 ? wsh[warp - 1] : 0);
+  *total = wsh[NW - 1];
+  __syncthreads();  // wsh free for the next scan
+  return res;
+}
+
+constexpr int kMaxFieldLines = 320;  // line starts held in shared memory: 264 NTSC, 314 PAL
+struct MapScratch {
+  double ll[kMaxFieldLines];  // the field's line starts from the first active line
+  int rf_s[kMaxRfDropouts], rf_e[kMaxRfDropouts];
+  int wsh[32];
+};
+
+// The field's active line starts into shared memory (no barrier).
+template <int THREADS>
+__device__ __forceinline__ void load_lines(const DropoutArgs& a, int f, MapScratch& m) {
+  const double* ll = a.ll + (size_t)f * a.lines_per_frame + a.active_line_start;
+  for (int i = threadIdx.x; i <= a.out_h; i += THREADS) m.ll[i] = ll[i];
+}
+
+// Entries of one span: TBC line l of the lines [sl, el] it touches, columns
+// [sx, ex).  False where the line gets no entry.
+__device__ __forceinline__ bool span_entry(const double* ll, int l, int sl, int el, double sa, double ea, int W,
+                                           int& sx, int& ex) {
+  const double l0 = ll[l], len = ll[l + 1] - l0;
+  if (len <= 0.0) return false;
+  sx = (l == sl) ? max(0, (int)((sa - l0) / len * (double)W)) : 0;
+  ex = (l == el) ? min(W, (int)((ea - l0) / len * (double)W + 0.999)) : W;
+  return ex > sx;
+}
+
+// Step 4 (whole CTA): merge start/end events (<= 30 samples apart), keep <= 128
+// spans, drop spans < 10 samples, map to TBC lines.  The state alternates from
+// "no dropout", so events 2i and 2i + 1 are the start and end of run i (the
+// last may lack its end: the range's end); a run joins the one before it when
+// its start lies within 30 samples of that one's end, so the spans are the
+// runs numbered by a prefix sum, and a span's entries go behind those of the
+// spans before it by another.  Latency bound (a few hundred events at most,
+// a few KB): one thread walking the events with each line search in global
+// memory took 0.5 ms for a field that reaches past the capture's end; the
+// searches now read shared memory, a thread per span.
+template <int THREADS>
+__device__ void map_events(const DropoutArgs& a, int f, const int* events, int ne, int s0, int s1, MapScratch& m) {
+  static_assert(THREADS >= kMaxRfDropouts, "a thread per span");
+  const int tid = threadIdx.x, H = a.out_h, W = a.out_w;
+  const int runs = (ne + 1) / 2;
+  auto start = [&](int i) { return s0 + (events[2 * i] >> 1) * 16; };
+  auto end = [&](int i) { return 2 * i + 1 < ne ? s0 + (events[2 * i + 1] >> 1) * 16 : s1; };
+  int nrf = 0;
+  for (int base = 0; base < runs; base += THREADS) {
+    const int i = base + tid;
+    const bool in = i < runs;
+    const bool first = in && (i == 0 || start(i) - end(i - 1) > 30);
+    int total;
+    const int g = nrf + block_excl_sum<THREADS>(first ? 1 : 0, m.wsh, &total) + (first ? 1 : 0) - 1;
+    if (in && g < kMaxRfDropouts) {
+      if (first) m.rf_s[g] = start(i);
+      if (i + 1 == runs || start(i + 1) - end(i) > 30) m.rf_e[g] = end(i);
+    }
+    nrf += total;
+  }
+  nrf = min(nrf, kMaxRfDropouts);
+  __syncthreads();
+  int sl = 0, el = -1, cnt = 0, sx, ex;
+  double sa = 0.0, ea = 0.0;
+  if (tid < nrf && m.rf_e[tid] - m.rf_s[tid] >= 10) {
+    sa = (double)m.rf_s[tid];
+    ea = (double)m.rf_e[tid];
+    sl = find_line(m.ll, H, sa);
+    if (sl >= 0) {
+      el = find_line(m.ll, H, ea - 1.0);
+      if (el < 0) el = H - 1;
+      for (int l = sl; l <= el; l++) cnt += span_entry(m.ll, l, sl, el, sa, ea, W, sx, ex) ? 1 : 0;
+    }
+  }
+  int n;
+  int k = block_excl_sum<THREADS>(cnt, m.wsh, &n);
   int* ol = a.do_lines + (size_t)f * kMaxDropouts;
   int* os = a.do_starts + (size_t)f * kMaxDropouts;
   int* oe = a.do_ends + (size_t)f * kMaxDropouts;
-  int nrf = 0, open = -1;
-  for (int e = 0; e < ne; e++) {
-    const int pos = s0 + (events[e] >> 1) * 16;
-    if (events[e] & 1) {
-      open = pos;
-    } else if (open >= 0) {
-      if (nrf > 0 && open - rf_e[nrf - 1] <= 30) rf_e[nrf - 1] = pos;
-      else if (nrf < kMaxRfDropouts) { rf_s[nrf] = open; rf_e[nrf] = pos; nrf++; }
-      open = -1;
-    }
-  }
-  if (open >= 0) {
-    if (nrf > 0 && open - rf_e[nrf - 1] <= 30) rf_e[nrf - 1] = s1;
-    else if (nrf < kMaxRfDropouts) { rf_s[nrf] = open; rf_e[nrf] = s1; nrf++; }
-  }
-  int n = 0;
-  for (int i = 0; i < nrf && n < kMaxDropouts; i++) {
-    if (rf_e[i] - rf_s[i] < 10) continue;
-    const double sa = (double)rf_s[i], ea = (double)rf_e[i];
-    const int sl = find_line(ll, als, H, sa);
-    if (sl < 0) continue;
-    int el = find_line(ll, als, H, ea - 1.0);
-    if (el < 0) el = H - 1;
-    for (int l = sl; l <= el && n < kMaxDropouts; l++) {
-      const double l0 = ll[als + l], l1 = ll[als + l + 1], len = l1 - l0;
-      if (len <= 0.0) continue;
-      const int sx = (l == sl) ? max(0, (int)((sa - l0) / len * (double)W)) : 0;
-      const int ex = (l == el) ? min(W, (int)((ea - l0) / len * (double)W + 0.999)) : W;
-      if (ex > sx) { ol[n] = l; os[n] = sx; oe[n] = ex; n++; }
-    }
-  }
-  a.do_count[f] = n;
-  return n;
+  if (cnt > 0)
+    for (int l = sl; l <= el && k < kMaxDropouts; l++)
+      if (span_entry(m.ll, l, sl, el, sa, ea, W, sx, ex)) {
+        ol[k] = l;
+        os[k] = sx;
+        oe[k] = ex;
+        k++;
+      }
+  if (tid == 0) a.do_count[f] = min(n, kMaxDropouts);
 }
 
-// Step 5 (one warp): conceal from the line above (below for line 0), groups of
-// 32 entries, every load of a column step before its stores.  Planes are
-// independent, so luma and chroma may be concealed in separate passes.
-__device__ void conceal(const DropoutArgs& a, int f, int n, int lane, bool luma, bool chroma) {
-  const int H = a.out_h, W = a.out_w;
+// Step 5: conceal from the line above (below for line 0).  The reference's
+// copy loop takes the entries 32 at a time, one column step after another,
+// every load of a step before its stores: entry d copies column c at step
+// c - sx_d.  So, inside a group of 32, column c of entry d holds what its
+// source row held at that step: the row's own pixel, or, where an entry e
+// covers c on that row and started further right (sx_e > sx_d, an earlier
+// step; the smallest such sx_e wrote last), what e's source row held at e's
+// step.  Each pixel's origin therefore follows from the entries alone, and
+// columns never mix: a thread takes a column through all groups in order,
+// the group's loads all in flight before its stores.  Latency bound; a warp
+// stepping through the columns took 0.7 us a step, 1.4 ms for a field with
+// 512 entries.
+struct ConcealEntry {
+  short line, src, sx, ex;
+  unsigned before;  // entries of the group on row src with a larger sx
+  unsigned after;   // entries of the group on the same line with a smaller sx (they write later)
+};
+static_assert(kMaxDropouts % 32 == 0, "whole groups");
+
+// The field's n entries with their links into shared memory (ends with a barrier).
+template <int THREADS>
+__device__ void conceal_entries(const DropoutArgs& a, int f, int n, ConcealEntry* ent) {
   const int* ol = a.do_lines + (size_t)f * kMaxDropouts;
   const int* os = a.do_starts + (size_t)f * kMaxDropouts;
   const int* oe = a.do_ends + (size_t)f * kMaxDropouts;
-  uint16_t* lf = a.luma + (size_t)f * H * W;
-  uint16_t* cf = a.chroma + (size_t)f * H * W;
-  for (int g = 0; g < n; g += 32) {
+  const int lane = threadIdx.x & 31;
+  for (int g = (threadIdx.x >> 5) * 32; g < n; g += THREADS) {
     const int d = g + lane;
-    int line = 0, sx = 0, ex = 0, src = H;
+    int line = -1, src = -2, sx = 0, ex = 0;
     if (d < n) {
-      line = ol[d]; sx = os[d]; ex = oe[d];
+      line = ol[d];
+      sx = os[d];
+      ex = oe[d];
       src = line > 0 ? line - 1 : line + 1;
+      if (src >= a.out_h) ex = sx;
     }
-    const int span = (d < n && src < H) ? ex - sx : 0;
-    int maxspan = span;
-    for (int off = 16; off > 0; off >>= 1) maxspan = max(maxspan, __shfl_xor_sync(0xffffffffu, maxspan, off));
-    for (int it = 0; it < maxspan; it++) {
-      const bool act = it < span;
-      uint16_t vl = 0, vc = 0;
-      if (act && luma) vl = lf[src * W + sx + it];
-      if (act && chroma) vc = cf[src * W + sx + it];
-      __syncwarp();
-      if (act && luma) lf[line * W + sx + it] = vl;
-      if (act && chroma) cf[line * W + sx + it] = vc;
-      __syncwarp();
+    unsigned before = 0, after = 0;
+    for (int e = 0; e < 32; e++) {
+      const int le = __shfl_sync(0xffffffffu, line, e), se = __shfl_sync(0xffffffffu, sx, e);
+      if (le == src && se > sx) before |= 1u << e;
+      if (le == line && se < sx) after |= 1u << e;
     }
+    ent[d] = ConcealEntry{(short)line, (short)src, (short)sx, (short)ex, before, after};
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ bool covers(const ConcealEntry& e, int c) { return c >= e.sx && c < e.ex; }
+
+// Column c of one plane through every group of entries.
+__device__ void conceal_column(const ConcealEntry* ent, int n, uint16_t* plane, int W, int c) {
+  for (int g = 0; g < n; g += 32) {
+    const int m = min(32, n - g);
+    uint16_t v[32];
+    unsigned act = 0;
+#pragma unroll
+    for (int d = 0; d < 32; d++) {
+      v[d] = 0;
+      if (d >= m) continue;
+      const ConcealEntry e = ent[g + d];
+      if (!covers(e, c)) continue;
+      bool last = true;  // no later write of the group to this pixel
+      for (unsigned w = e.after; w; w &= w - 1) last = last && !covers(ent[g + __ffs(w) - 1], c);
+      if (!last) continue;
+      act |= 1u << d;
+      int row = e.src;
+      for (unsigned w = e.before; w;) {
+        int best = -1, bsx = 1 << 30;
+        for (; w; w &= w - 1) {
+          const int k = __ffs(w) - 1;
+          if (covers(ent[g + k], c) && ent[g + k].sx < bsx) {
+            best = k;
+            bsx = ent[g + k].sx;
+          }
+        }
+        if (best >= 0) {
+          row = ent[g + best].src;
+          w = ent[g + best].before;
+        }
+      }
+      v[d] = plane[row * W + c];
+    }
+#pragma unroll
+    for (int d = 0; d < 32; d++)
+      if (act >> d & 1u) plane[ent[g + d].line * W + c] = v[d];
   }
 }
 
@@ -154,12 +279,13 @@ __global__ void __launch_bounds__(kThreadsD) dropout_kernel(DropoutArgs a) {
   __shared__ int ev_off[kThreadsD];
   __shared__ int events[kMaxEvents];  // block index * 2 + (1 = start, 0 = end)
   __shared__ int n_events;
-  __shared__ int rf_s[kMaxRfDropouts], rf_e[kMaxRfDropouts];
-  __shared__ int n_entries;
+  __shared__ MapScratch map;
+  __shared__ ConcealEntry ent[kMaxDropouts];
   __shared__ double down_s;
   const int f = blockIdx.x;
   const int tid = threadIdx.x;
   if (tid == 0) down_s = down_threshold(a, f);
+  load_lines<kThreadsD>(a, f, map);
   int s0, s1;
   active_range(a, f, s0, s1);
   __syncthreads();
@@ -215,9 +341,16 @@ __global__ void __launch_bounds__(kThreadsD) dropout_kernel(DropoutArgs a) {
     else if (cls[b] == 1 && st) { st = 0; if (k < kMaxEvents) events[k] = b * 2; k++; }
   }
   __syncthreads();
-  if (tid == 0) n_entries = map_events(a, f, events, min(n_events, kMaxEvents), s0, s1, rf_s, rf_e);
-  __syncthreads();
-  if (tid < 32) conceal(a, f, n_entries, tid, true, true);
+  map_events<kThreadsD>(a, f, events, min(n_events, kMaxEvents), s0, s1, map);
+  __syncthreads();  // the entries and their count, written by this CTA
+  const int n = a.do_count[f];
+  if (n <= 0) return;  // whole CTA
+  conceal_entries<kThreadsD>(a, f, n, ent);
+  const size_t F = (size_t)a.out_h * a.out_w;
+  for (int c = tid; c < a.out_w; c += kThreadsD) {
+    conceal_column(ent, n, a.luma + f * F, a.out_w, c);
+    conceal_column(ent, n, a.chroma + f * F, a.out_w, c);
+  }
 }
 
 // --------------------------------------------------------------- two-pass form
@@ -273,34 +406,8 @@ __global__ void __launch_bounds__(kThreadsD) dropout_class_kernel(const __grid_c
   a.cls[(size_t)f * a.max_blocks + b] = block_class(sum, n, down, down * 1.25);
 }
 
-// Block-wide exclusive scans over kThreadsScan threads (warp shuffles, then
-// the warp totals).  wsh holds 32 ints; every thread must call.
-__device__ __forceinline__ int block_excl_sum(int v, int* wsh, int* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int NW = kThreadsScan / 32;
-  int x = v;
-  for (int off = 1; off < 32; off <<= 1) {
-    const int o = __shfl_up_sync(0xffffffffu, x, off);
-    if (lane >= off) x += o;
-  }
-  if (lane == 31) wsh[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    int w = lane < NW ? wsh[lane] : 0;
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, w, off);
-      if (lane >= off) w += o;
-    }
-    if (lane < NW) wsh[lane] = w;  // inclusive warp prefix
-  }
-  __syncthreads();
-  const int res = x - v + (warp > 0 ? wsh[warp - 1] : 0);
-  *total = wsh[NW - 1];
-  __syncthreads();  // wsh free for the next scan
-  return res;
-}
-
 // "Last decisive class" prefix: combine(left, right) = right != -1 ? right : left.
+// Block-wide over kThreadsScan threads; wsh holds 32 ints, every thread must call.
 __device__ __forceinline__ int block_excl_last(int v, int* wsh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NW = kThreadsScan / 32;
@@ -329,7 +436,10 @@ __device__ __forceinline__ int block_excl_last(int v, int* wsh) {
 
 // One CTA per field: class bytes back from L2 into shared memory, then the
 // hysteresis scan, event list, mapping and luma concealment (chroma is
-// concealed by dropout_chroma_kernel once the chroma planes are final).
+// concealed by conceal_chroma_kernel once the chroma planes are final).  The
+// luma is concealed here rather than in a kernel of its own: the chroma lines
+// fill the SMs by then, and one more low-priority launch held the luma copy
+// of a 40-field capture back by 18 us (1,617 -> 1,634 us a capture).
 template <class Src>
 __global__ void __launch_bounds__(kThreadsScan) dropout_scan_kernel(const __grid_constant__ Src src) {
   const DropoutArgs& a = src.get();
@@ -338,8 +448,8 @@ __global__ void __launch_bounds__(kThreadsScan) dropout_scan_kernel(const __grid
   extern __shared__ uint4 cls4[];  // [a.max_blocks / 16]
   __shared__ int wsh[32];
   __shared__ int events[kMaxEvents];
-  __shared__ int rf_s[kMaxRfDropouts], rf_e[kMaxRfDropouts];
-  __shared__ int n_entries;
+  __shared__ MapScratch map;
+  __shared__ ConcealEntry ent[kMaxDropouts];
   const unsigned char* cls = reinterpret_cast<const unsigned char*>(cls4);
   const int f = blockIdx.x, tid = threadIdx.x;
   int s0, s1;
@@ -351,6 +461,7 @@ __global__ void __launch_bounds__(kThreadsScan) dropout_scan_kernel(const __grid
   const int nb = min((s1 - s0 + 15) / 16, a.max_blocks);
   const uint4* cls_in = reinterpret_cast<const uint4*>(a.cls + (size_t)f * a.max_blocks);
   for (int i = tid; i < (nb + 15) / 16; i += kThreadsScan) cls4[i] = cls_in[i];
+  load_lines<kThreadsScan>(a, f, map);
   __syncthreads();
   const int per = (nb + kThreadsScan - 1) / kThreadsScan;
   const int b_lo = min(nb, tid * per), b_hi = min(nb, b_lo + per);
@@ -365,27 +476,43 @@ __global__ void __launch_bounds__(kThreadsScan) dropout_scan_kernel(const __grid
     else if (cls[b] == 1 && st) { st = 0; cnt++; }
   }
   int n_events;
-  int k = block_excl_sum(cnt, wsh, &n_events);
+  int k = block_excl_sum<kThreadsScan>(cnt, wsh, &n_events);
   st = st_in;
   for (int b = b_lo; b < b_hi; b++) {
     if (cls[b] == 0 && !st) { st = 1; if (k < kMaxEvents) events[k] = b * 2 + 1; k++; }
     else if (cls[b] == 1 && st) { st = 0; if (k < kMaxEvents) events[k] = b * 2; k++; }
   }
   __syncthreads();
-  if (tid == 0) n_entries = map_events(a, f, events, min(n_events, kMaxEvents), s0, s1, rf_s, rf_e);
-  __syncthreads();
-  if (tid < 32) conceal(a, f, n_entries, tid, true, false);
+  if (n_events == 0) {
+    if (tid == 0) a.do_count[f] = 0;
+    return;  // whole CTA
+  }
+  map_events<kThreadsScan>(a, f, events, min(n_events, kMaxEvents), s0, s1, map);
+  __syncthreads();  // the entries and their count, written by this CTA
+  const int n = a.do_count[f];
+  if (n <= 0) return;  // whole CTA
+  conceal_entries<kThreadsScan>(a, f, n, ent);
+  uint16_t* plane = a.luma + (size_t)f * a.out_h * a.out_w;
+  for (int c = tid; c < a.out_w; c += kThreadsScan) conceal_column(ent, n, plane, a.out_w, c);
 }
 
-// One warp per field: chroma concealment from the entries the scan kernel wrote.
+// Chroma concealment of fields [f0, f0 + nf) from the entries the scan kernel
+// wrote: grid (fields, column strips), a thread per column, so that a field
+// with many entries is spread over several SMs.
+constexpr int kConcealThreads = 256;
 template <class Src>
-__global__ void dropout_chroma_kernel(const __grid_constant__ Src src, int f0, int nf) {
+__global__ void __launch_bounds__(kConcealThreads) conceal_chroma_kernel(const __grid_constant__ Src src, int f0, int nf) {
   const DropoutArgs& a = src.get();
+  const int f = f0 + blockIdx.x;
+  if (f >= f0 + nf || f >= a.fields) return;  // whole CTA
   chain_wait();
-  const int f = f0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (f >= f0 + nf || f >= a.fields) return;  // whole warp
+  __shared__ ConcealEntry ent[kMaxDropouts];
   const int n = min(max(a.do_count[f], 0), kMaxDropouts);
-  conceal(a, f, n, threadIdx.x & 31, false, true);
+  if (n == 0) return;  // whole CTA
+  conceal_entries<kConcealThreads>(a, f, n, ent);
+  const int c = blockIdx.y * kConcealThreads + threadIdx.x;
+  uint16_t* plane = a.chroma + (size_t)f * a.out_h * a.out_w;
+  if (c < a.out_w) conceal_column(ent, n, plane, a.out_w, c);
 }
 
 }  // namespace
@@ -407,6 +534,12 @@ size_t dropout_class_bytes_per_field(int spp) { return (size_t)(((spp + 15) / 16
 
 namespace {
 template <class S>
+void conceal_launch(const S& src, const DropoutArgs& a, int portions, int f0, int nf, cudaStream_t st) {
+  const int strips = (a.out_w + kConcealThreads - 1) / kConcealThreads;
+  launch_chained(conceal_chroma_kernel<S>, dim3(nf, strips, portions), dim3(kConcealThreads), 0, st, src, f0, nf);
+}
+
+template <class S>
 void two_pass_launch(const S& src, const DropoutArgs& a, int portions, int max_fields, cudaStream_t st) {
   dim3 grid((a.max_blocks + kThreadsD - 1) / kThreadsD, max_fields, portions);
   launch_chained(dropout_class_kernel<S>, grid, dim3(kThreadsD), 0, st, src);
@@ -415,12 +548,6 @@ void two_pass_launch(const S& src, const DropoutArgs& a, int portions, int max_f
   launch_chained(dropout_scan_kernel<S>, dim3(max_fields, 1, portions), dim3(kThreadsScan), smem, st, src);
 }
 
-template <class S>
-void conceal_launch(const S& src, int portions, int f0, int nf, cudaStream_t st) {
-  const int threads = 128;
-  launch_chained(dropout_chroma_kernel<S>, dim3((nf * 32 + threads - 1) / threads, 1, portions), dim3(threads), 0, st,
-                 src, f0, nf);
-}
 }  // namespace
 
 void launch_dropouts_two_pass(const DropoutArgs& a, cudaStream_t st) {
@@ -430,7 +557,7 @@ void launch_dropouts_two_pass(const DropoutArgs& a, cudaStream_t st) {
 
 void launch_dropout_conceal_chroma(const DropoutArgs& a, int f0, int nf, cudaStream_t st) {
   if (nf <= 0 || f0 < 0 || f0 >= a.fields) return;
-  conceal_launch(ArgsOne<DropoutArgs>{a}, 1, f0, nf, st);
+  conceal_launch(ArgsOne<DropoutArgs>{a}, a, 1, f0, nf, st);
 }
 
 void launch_dropouts_two_pass_many(const ArgsMany<DropoutArgs>& p, int portions, int max_fields, cudaStream_t st) {
@@ -439,7 +566,7 @@ void launch_dropouts_two_pass_many(const ArgsMany<DropoutArgs>& p, int portions,
 
 void launch_dropout_conceal_chroma_many(const ArgsMany<DropoutArgs>& p, int portions, int max_fields,
                                         cudaStream_t st) {
-  if (portions > 0 && max_fields > 0) conceal_launch(p, portions, 0, max_fields, st);
+  if (portions > 0 && max_fields > 0) conceal_launch(p, p.a[0], portions, 0, max_fields, st);
 }
 
 }  // namespace cuvhs
