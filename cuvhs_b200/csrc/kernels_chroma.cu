@@ -23,7 +23,11 @@ namespace {
 
 // 16 elements per thread, 1024 threads at 64 registers each (spill-free since
 // the inverse transform takes an opaque thread index); 32 elements with 512
-// threads at 128 registers is also spill-free but measured 9% slower.
+// threads at 128 registers is also spill-free but measured 9% slower.  The
+// 16384-point transform fills the register file and 139 KB of shared memory, so
+// one CTA runs on an SM and its own warps must cover each other: with packed
+// arithmetic and one barrier a pass 139 -> 132 us (40 fields at 28 MHz; issue
+// 42%, FP32 pipe 37%, shared memory 33%).
 constexpr int kElemsC = 16;
 constexpr int kThreadsC = Design::kNc / kElemsC;
 // Line kernel geometry: a line pair (two lines in one complex transform) per
@@ -83,13 +87,11 @@ __global__ void __launch_bounds__(kThreadsC, 1) prefilter_kernel(const __grid_co
       v[q] = make_float2(v0, v1);
     }
   }
-  RegFFT<N, E>::run<false>(v, sm, a.tw_c, t);
+  RegFFT<N>::run<false>(v, sm, a.tw_c, t);
+  float g[E];
 #pragma unroll
-  for (int q = 0; q < E; q++) {
-    const float g = __ldg(&a.gc[t + T * q]);
-    v[q] = make_float2(v[q].x * g, v[q].y * g);
-  }
-  RegFFT<N, E>::run<true>(v, sm, a.tw_c_inv, opaque_index(t));
+  for (int q = 0; q < E; q++) g[q] = __ldg(&a.gc[t + T * q]);
+  RegFFT<N>::run_gains<true>(v, g, sm, a.tw_c_inv, opaque_index(t));
   float* out = a.pre + (size_t)f * a.spp;
 #pragma unroll
   for (int q = 0; q < E; q++) {

@@ -1,48 +1,76 @@
-// Register-resident block FFT for one CTA of T = N/E threads (sm_100a), E = 16
-// or 32 elements per thread.
+// Register-resident block FFT for one CTA of T = N/16 threads (sm_100a).
 //
-// Thread t owns elements t + T*q, q = 0..E-1, of an N-point transform, both on
-// entry (natural-order input) and on exit (natural-order output): Stockham
-// passes of radix 16 (and one final radix 2/4/8 when N is not a power of 16)
-// exchange data through a padded shared buffer between passes, but the first
+// Thread t owns elements t + T*q, q = 0..15, of an N-point transform, both on
+// entry (natural-order input) and on exit (natural-order output): radix-16
+// passes (and one final radix 2/4 when N is not a power of 16) exchange data
+// through a padded shared buffer between passes, but the first
 // pass reads its inputs from registers and the last pass leaves its outputs in
 // registers.  Since the output layout equals the input layout, a forward
 // transform, a per-bin multiply and an inverse transform chain without any
 // shared-memory round trip at the seams, and inputs/outputs move between HBM
 // and registers with coalesced accesses (consecutive threads, consecutive
 // elements).  Twiddles: the per-pass table of smem_fft.cuh (coalesced loads).
+//
+// The butterflies and twiddles are those of the Stockham passes of
+// smem_fft.cuh, but a pass between the first and the last writes each output
+// back where its butterfly read an input.  So a warp goes from its reads
+// through the arithmetic to its writes without waiting for the others, one
+// barrier a pass instead of two, and warps in different parts of a pass fill
+// the FP32 pipe, the load/store unit and shared memory side by side.  (With a
+// barrier between reads and writes all warps of a CTA met in the same unit:
+// issue at 45-47% of cycles with every unit below 37%.)  The logical index i
+// of pass p lies at: pass 2, i; pass 3, i with its two lowest base-16 digits'
+// butterfly undone, and so on -- in each pass a constant stride for a
+// butterfly's slots and 16 consecutive elements for 16 consecutive threads,
+// hence no bank conflicts.
 #pragma once
 #include "smem_fft.cuh"
 
 namespace cuvhs {
 
-template <int N, int E = 16>
+template <int N>
 struct RegFFT {
-  static_assert(E == 16 || E == 32, "16 or 32 elements per thread");
-  static constexpr int T = N / E;
-  static constexpr int G = E / 16;  // first-pass radix-16 butterflies per thread
+  static_assert(N == 4096 || N == 8192 || N == 16384, "three radix-16 passes and a last one of 1, 2 or 4");
+  static constexpr int T = N / 16;
 
-  // One pass of radix R at span NS (> 1).  v holds the E values this thread
-  // reads; LAST leaves the results in v in the t + T*q layout.
+  // Padded location of slot 0 of thread t's (first) butterfly in the pass of
+  // span NS, and the strides from slot to slot and from butterfly to butterfly
+  // (logical inputs t + T*b + r*N/R).
+  template <int NS>
+  __device__ __forceinline__ static int place(int t) {
+    const int lo = t & 15, mid = ((t >> 4) & 15) * T, hi = t >> 8;
+    if constexpr (NS == 16) return pidx(t);
+    else if constexpr (NS == 256) return pidx(hi * 16 + lo + mid);
+    else return pidx(hi * (T / 16) + lo + mid);
+  }
+  template <int NS>
+  __host__ __device__ static constexpr int slot_stride() {
+    return NS == 16 ? fft_pad(T) : (NS == 256 ? fft_pad(T / 16) : 17);
+  }
+  template <int NS>
+  __host__ __device__ static constexpr int butterfly_stride() {  // the last pass of N > 4096 has several
+    return fft_pad((T / 256) * (T / 16));
+  }
+
+  // One pass of radix R at span NS (> 1).  LAST leaves the results in v in the
+  // t + T*q layout.
   template <int NS, bool INV, bool LAST>
-  __device__ __forceinline__ static void pass(float2 (&v)[E], float2* s, const float2* __restrict__ tw, int t) {
+  __device__ __forceinline__ static void pass(float2 (&v)[16], float2* s, const float2* __restrict__ tw, int t) {
     constexpr int R = fft_radix(N, NS);
-    constexpr int B = E / R;  // butterflies per thread
-    // inputs are twiddled as they are read, so only the E values stay live
-    // across the barrier
+    constexpr int B = 16 / R;  // butterflies per thread
+    static_assert(LAST || B == 1, "only the last pass has a smaller radix");
+    float2* p = s + place<NS>(t);
     float2 w[B][R];
 #pragma unroll
     for (int b = 0; b < B; b++) {
-      const int j = t + T * b;
-      const int k = j & (NS - 1);
+      const int k = (t + T * b) & (NS - 1);
       const float2* twp = tw + (NS - 16) + k;
-      w[b][0] = s[pidx(j)];
+      w[b][0] = p[b * butterfly_stride<NS>()];
 #pragma unroll
-      for (int r = 1; r < R; r++) w[b][r] = cmul_tw<INV>(s[pidx(j + r * (N / R))], __ldg(&twp[(r - 1) * NS]));
+      for (int r = 1; r < R; r++)
+        w[b][r] = cmul_tw<INV>(p[b * butterfly_stride<NS>() + r * slot_stride<NS>()], __ldg(&twp[(r - 1) * NS]));
+      dft<R, INV>(w[b]);
     }
-    __syncthreads();  // every read done before this pass (or the caller) overwrites
-#pragma unroll
-    for (int b = 0; b < B; b++) dft<R, INV>(w[b]);
     if constexpr (LAST) {
 #pragma unroll
       for (int b = 0; b < B; b++)
@@ -50,23 +78,16 @@ struct RegFFT {
         for (int r = 0; r < R; r++) v[b + B * r] = w[b][dft_slot<R>(r)];
     } else {
 #pragma unroll
-      for (int b = 0; b < B; b++) {
-        const int j = t + T * b;
-        const int k = j & (NS - 1);
-        const int base = (j / NS) * NS * R + k;
-#pragma unroll
-        for (int r = 0; r < R; r++) s[pidx(base + r * NS)] = w[b][dft_slot<R>(r)];
-      }
+      for (int r = 0; r < R; r++) p[r * slot_stride<NS>()] = w[0][dft_slot<R>(r)];
       __syncthreads();
     }
   }
 
   template <int NS, bool INV>
-  __device__ __forceinline__ static void rest(float2 (&v)[E], float2* s, const float2* __restrict__ tw, int t) {
-    constexpr int R = fft_radix(N, NS);
-    constexpr bool LAST = NS * R >= N;
+  __device__ __forceinline__ static void rest(float2 (&v)[16], float2* s, const float2* __restrict__ tw, int t) {
+    constexpr bool LAST = NS * fft_radix(N, NS) >= N;
     pass<NS, INV, LAST>(v, s, tw, t);
-    if constexpr (!LAST) rest<NS * R, INV>(v, s, tw, t);
+    if constexpr (!LAST) rest<NS * fft_radix(N, NS), INV>(v, s, tw, t);
   }
 
   // Two independent transforms of the same direction in lockstep: v1 with
@@ -74,28 +95,26 @@ struct RegFFT {
   // waits on one barrier for both, and has twice the independent arithmetic;
   // every value is computed exactly as by two run() calls.
   template <int NS, bool INV, bool LAST>
-  __device__ __forceinline__ static void pass2(float2 (&v1)[E], float2* s1, float2 (&v2)[E], float2* s2,
+  __device__ __forceinline__ static void pass2(float2 (&v1)[16], float2* s1, float2 (&v2)[16], float2* s2,
                                                const float2* __restrict__ tw, int t) {
     constexpr int R = fft_radix(N, NS);
-    constexpr int B = E / R;
+    constexpr int B = 16 / R;
+    static_assert(LAST || B == 1, "only the last pass has a smaller radix");
+    const int at = place<NS>(t);
     float2 w1[B][R], w2[B][R];
 #pragma unroll
     for (int b = 0; b < B; b++) {
-      const int j = t + T * b;
-      const int k = j & (NS - 1);
+      const int k = (t + T * b) & (NS - 1);
       const float2* twp = tw + (NS - 16) + k;
-      w1[b][0] = s1[pidx(j)];
-      w2[b][0] = s2[pidx(j)];
+      const int o = at + b * butterfly_stride<NS>();
+      w1[b][0] = s1[o];
+      w2[b][0] = s2[o];
 #pragma unroll
       for (int r = 1; r < R; r++) {
         const float2 c = __ldg(&twp[(r - 1) * NS]);
-        w1[b][r] = cmul_tw<INV>(s1[pidx(j + r * (N / R))], c);
-        w2[b][r] = cmul_tw<INV>(s2[pidx(j + r * (N / R))], c);
+        w1[b][r] = cmul_tw<INV>(s1[o + r * slot_stride<NS>()], c);
+        w2[b][r] = cmul_tw<INV>(s2[o + r * slot_stride<NS>()], c);
       }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < B; b++) {
       dft<R, INV>(w1[b]);
       dft<R, INV>(w2[b]);
     }
@@ -109,77 +128,70 @@ struct RegFFT {
         }
     } else {
 #pragma unroll
-      for (int b = 0; b < B; b++) {
-        const int j = t + T * b;
-        const int k = j & (NS - 1);
-        const int base = (j / NS) * NS * R + k;
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          s1[pidx(base + r * NS)] = w1[b][dft_slot<R>(r)];
-          s2[pidx(base + r * NS)] = w2[b][dft_slot<R>(r)];
-        }
+      for (int r = 0; r < R; r++) {
+        s1[at + r * slot_stride<NS>()] = w1[0][dft_slot<R>(r)];
+        s2[at + r * slot_stride<NS>()] = w2[0][dft_slot<R>(r)];
       }
       __syncthreads();
     }
   }
 
   template <int NS, bool INV>
-  __device__ __forceinline__ static void rest2(float2 (&v1)[E], float2* s1, float2 (&v2)[E], float2* s2,
+  __device__ __forceinline__ static void rest2(float2 (&v1)[16], float2* s1, float2 (&v2)[16], float2* s2,
                                                const float2* __restrict__ tw, int t) {
-    constexpr int R = fft_radix(N, NS);
-    constexpr bool LAST = NS * R >= N;
+    constexpr bool LAST = NS * fft_radix(N, NS) >= N;
     pass2<NS, INV, LAST>(v1, s1, v2, s2, tw, t);
-    if constexpr (!LAST) rest2<NS * R, INV>(v1, s1, v2, s2, tw, t);
+    if constexpr (!LAST) rest2<NS * fft_radix(N, NS), INV>(v1, s1, v2, s2, tw, t);
   }
 
   // run() on two transforms at once (see pass2); s1 and s2 may be in use by
   // the caller until this call.
   template <bool INV>
-  __device__ __forceinline__ static void run2(float2 (&v1)[E], float2* s1, float2 (&v2)[E], float2* s2,
+  __device__ __forceinline__ static void run2(float2 (&v1)[16], float2* s1, float2 (&v2)[16], float2* s2,
                                               const float2* __restrict__ tw, int t) {
-    static_assert(N >= 256 && (N & (N - 1)) == 0, "power of two >= 256");
-    float2 w1[G][16], w2[G][16];
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-#pragma unroll
-      for (int r = 0; r < 16; r++) {
-        w1[g][r] = v1[g + G * r];
-        w2[g][r] = v2[g + G * r];
-      }
-      dft<16, INV>(w1[g]);
-      dft<16, INV>(w2[g]);
-    }
+    dft<16, INV>(v1);
+    dft<16, INV>(v2);
     __syncthreads();
 #pragma unroll
-    for (int g = 0; g < G; g++)
-#pragma unroll
-      for (int r = 0; r < 16; r++) {
-        s1[pidx(16 * (t + T * g) + r)] = w1[g][dft_slot<16>(r)];
-        s2[pidx(16 * (t + T * g) + r)] = w2[g][dft_slot<16>(r)];
-      }
+    for (int r = 0; r < 16; r++) {
+      s1[pidx(16 * t + r)] = v1[dft_slot<16>(r)];
+      s2[pidx(16 * t + r)] = v2[dft_slot<16>(r)];
+    }
     __syncthreads();
     rest2<16, INV>(v1, s1, v2, s2, tw, t);
   }
 
   // Transform v in place.  The buffer s (fft_pad(N) float2) may be in use by
-  // the caller until this call: the first write waits on a barrier.
+  // the caller until this call: the first write waits on a barrier.  On return
+  // other threads may still be reading s: a barrier comes before its next use.
   template <bool INV>
-  __device__ __forceinline__ static void run(float2 (&v)[E], float2* s, const float2* __restrict__ tw, int t) {
-    static_assert(N >= 256 && (N & (N - 1)) == 0, "power of two >= 256");
-    // pass NS = 1: butterfly t + T*g reads elements t + T*(g + G*r), all
-    // held by this thread (slots g + G*r)
-    float2 w[G][16];
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-#pragma unroll
-      for (int r = 0; r < 16; r++) w[g][r] = v[g + G * r];
-      dft<16, INV>(w[g]);
-    }
+  __device__ __forceinline__ static void run(float2 (&v)[16], float2* s, const float2* __restrict__ tw, int t) {
+    // pass NS = 1: butterfly t reads elements t + T*r, all held by this thread
+    dft<16, INV>(v);
+    after_first<INV>(v, s, tw, t);
+  }
+
+  // run() of an input whose upper half (slots 8..15) is zero; v[8..15] is not read.
+  template <bool INV>
+  __device__ __forceinline__ static void run_half(float2 (&v)[16], float2* s, const float2* __restrict__ tw, int t) {
+    dft16_half<INV>(v);
+    after_first<INV>(v, s, tw, t);
+  }
+
+  // run() of g[q] * v[q], real gains.
+  template <bool INV>
+  __device__ __forceinline__ static void run_gains(float2 (&v)[16], const float (&g)[16], float2* s,
+                                                   const float2* __restrict__ tw, int t) {
+    dft16_gains<INV>(v, g);
+    after_first<INV>(v, s, tw, t);
+  }
+
+  template <bool INV>
+  __device__ __forceinline__ static void after_first(float2 (&v)[16], float2* s, const float2* __restrict__ tw,
+                                                     int t) {
     __syncthreads();
 #pragma unroll
-    for (int g = 0; g < G; g++)
-#pragma unroll
-      for (int r = 0; r < 16; r++) s[pidx(16 * (t + T * g) + r)] = w[g][dft_slot<16>(r)];
+    for (int r = 0; r < 16; r++) s[pidx(16 * t + r)] = v[dft_slot<16>(r)];
     __syncthreads();
     rest<16, INV>(v, s, tw, t);
   }

@@ -9,8 +9,13 @@
 // rounded once to FP32: pass NS (>= 16) stores W_{NS*R}^{r*k} at
 // (NS - 16) + (r - 1) * NS + k, so a warp's twiddle loads (consecutive k) are
 // contiguous.  fft_twiddle_count(N) entries in all.
+//
+// Complex arithmetic is packed (packed.cuh): a complex value is one register
+// pair, an addition one instruction, a product two.  The products' rounding is
+// written out (fma(a, b, -(c*d)), fma(a, b, c*d)) instead of left to the
+// compiler, so the same transform rounds alike in every kernel.
 #pragma once
-#include <cuda_runtime.h>
+#include "packed.cuh"
 
 namespace cuvhs {
 
@@ -36,15 +41,15 @@ __host__ __device__ constexpr int fft_twiddle_count(int N) {
 }
 __device__ __forceinline__ int pidx(int i) { return i + (i >> 4); }
 
+// a * w (forward) or a * conj(w) (inverse)
 template <bool INV>
 __device__ __forceinline__ float2 cmul_tw(float2 a, float2 w) {
-  // a * w (forward) or a * conj(w) (inverse)
-  if (INV) return make_float2(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
-  return make_float2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
+  if (INV) return parts(f2_fma(f2(a), f2(w.x, w.x), f2(a.y, a.x) * f2(w.y, -w.y)));
+  return parts(f2_fma(f2(a.x, a.x), f2(w), f2(a.y, a.y) * f2(-w.y, w.x)));
 }
 
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return parts(f2(a) + f2(b)); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return parts(f2(a) - f2(b)); }
 
 // multiply by -i (forward) / +i (inverse)
 template <bool INV>
@@ -74,7 +79,8 @@ __device__ __forceinline__ float2 rot(float2 v) {
   if (m16 == 12) return mul_mi<!INV>(v);
   const float c = Root16::c[m16];
   const float s = INV ? Root16::s[m16] : -Root16::s[m16];
-  return make_float2(v.x * c - v.y * s, v.x * s + v.y * c);
+  if (!INV && (m16 == 1 || m16 == 3)) return parts(f2_fma(f2(v), f2(c, c), f2(v.y, v.x) * f2(-s, s)));
+  return parts(f2_fma(f2(v.x, v.x), f2(c, s), f2(v.y, v.y) * f2(-s, c)));
 }
 
 template <bool INV>
@@ -100,6 +106,22 @@ __host__ __device__ constexpr int dft_slot(int r) {
   return R == 16 ? 4 * (r & 3) + (r >> 2) : (R == 8 ? 2 * (r & 3) + (r >> 2) : r);
 }
 
+// Second half of dft<16>: the inner turns and the dft4 over n2.
+template <bool INV>
+__device__ __forceinline__ void dft16_second(float2* v) {
+  v[4 + 1] = rot<16, 1, INV>(v[4 + 1]);
+  v[4 + 2] = rot<16, 2, INV>(v[4 + 2]);
+  v[4 + 3] = rot<16, 3, INV>(v[4 + 3]);
+  v[8 + 1] = rot<16, 2, INV>(v[8 + 1]);
+  v[8 + 2] = rot<16, 4, INV>(v[8 + 2]);
+  v[8 + 3] = rot<16, 6, INV>(v[8 + 3]);
+  v[12 + 1] = rot<16, 3, INV>(v[12 + 1]);
+  v[12 + 2] = rot<16, 6, INV>(v[12 + 2]);
+  v[12 + 3] = rot<16, 9, INV>(v[12 + 3]);
+#pragma unroll
+  for (int k1 = 0; k1 < 4; k1++) dft4<INV>(v[4 * k1], v[4 * k1 + 1], v[4 * k1 + 2], v[4 * k1 + 3]);
+}
+
 template <int R, bool INV>
 __device__ __forceinline__ void dft(float2* v) {
   if constexpr (R == 2) {
@@ -120,18 +142,44 @@ __device__ __forceinline__ void dft(float2* v) {
     // bin k1 + 4 k2 lands in v[4 k1 + k2]
 #pragma unroll
     for (int n2 = 0; n2 < 4; n2++) dft4<INV>(v[n2], v[4 + n2], v[8 + n2], v[12 + n2]);
-    v[4 + 1] = rot<16, 1, INV>(v[4 + 1]);
-    v[4 + 2] = rot<16, 2, INV>(v[4 + 2]);
-    v[4 + 3] = rot<16, 3, INV>(v[4 + 3]);
-    v[8 + 1] = rot<16, 2, INV>(v[8 + 1]);
-    v[8 + 2] = rot<16, 4, INV>(v[8 + 2]);
-    v[8 + 3] = rot<16, 6, INV>(v[8 + 3]);
-    v[12 + 1] = rot<16, 3, INV>(v[12 + 1]);
-    v[12 + 2] = rot<16, 6, INV>(v[12 + 2]);
-    v[12 + 3] = rot<16, 9, INV>(v[12 + 3]);
-#pragma unroll
-    for (int k1 = 0; k1 < 4; k1++) dft4<INV>(v[4 * k1], v[4 * k1 + 1], v[4 * k1 + 2], v[4 * k1 + 3]);
+    dft16_second<INV>(v);
   }
+}
+
+// dft<16, INV> of g[i] * v[i] with real gains g, the products fused into the
+// first additions.
+template <bool INV>
+__device__ __forceinline__ void dft16_gains(float2* v, const float* g) {
+#pragma unroll
+  for (int n2 = 0; n2 < 4; n2++) {
+    const F2 g0 = f2(g[n2], g[n2]), g1 = f2(g[4 + n2], g[4 + n2]);
+    const F2 g2 = f2(g[8 + n2], g[8 + n2]), g3 = f2(g[12 + n2], g[12 + n2]);
+    const F2 a0 = f2(v[n2]), a1 = f2(v[4 + n2]), a2 = f2(v[8 + n2]), a3 = f2(v[12 + n2]);
+    const F2 n2_ = f2(-v[8 + n2].x, -v[8 + n2].y), n3_ = f2(-v[12 + n2].x, -v[12 + n2].y);
+    const F2 t0 = f2_fma(a0, g0, a2 * g2);
+    const F2 t2 = f2_fma(a1, g1, a3 * g3);
+    const F2 t1 = f2_fma(a0, g0, n2_ * g2);
+    const F2 t3 = f2(mul_mi<INV>(parts(f2_fma(a1, g1, n3_ * g3))));
+    v[n2] = parts(t0 + t2);
+    v[8 + n2] = parts(t0 - t2);
+    v[4 + n2] = parts(t1 + t3);
+    v[12 + n2] = parts(t1 - t3);
+  }
+  dft16_second<INV>(v);
+}
+
+// dft<16, INV> of an input whose upper half v[8..15] is zero (not read).
+template <bool INV>
+__device__ __forceinline__ void dft16_half(float2* v) {
+#pragma unroll
+  for (int n2 = 0; n2 < 4; n2++) {
+    const float2 a = v[n2], b = v[4 + n2], c = mul_mi<INV>(b);
+    v[n2] = cadd(a, b);
+    v[4 + n2] = cadd(a, c);
+    v[8 + n2] = csub(a, b);
+    v[12 + n2] = csub(a, c);
+  }
+  dft16_second<INV>(v);
 }
 
 template <int THREADS>
