@@ -70,6 +70,7 @@ struct Design {
   double a_tail = 0;            // relative l2 energy outside the kept support
   float rot_re = 1, rot_im = 0;  // e^{-i d0}: nominal carrier phase step removed before atan2
   double d0 = 0;                 // nominal phase step (rad/sample) at ire0
+  float wrap = 0;                // largest FP32 step r with r + d0 (FP32) at most pi: above it the step wraps
   float demod_scale = 0;         // fs / 2pi
   float demod_offset = 0;        // d0 * fs/2pi - ire0 (Hz)
   // K1b: demod -> video (real part) + sync (imag part)
@@ -155,7 +156,7 @@ struct DemodArgs {
   const float2* tw_a_inv;
   const float2* tw_b_inv;
   int a_pos, a_out, b_pos, b_out;
-  float rot_re, rot_im, d0, demod_scale, demod_offset;
+  float rot_re, rot_im, wrap, demod_scale, demod_offset;
   float corr_video, corr_sync;
   float* dem;      // [T*spp] demod - ire0 (Hz)
   float* env;      // [T*spp] |analytic|

@@ -279,6 +279,16 @@ void Design::build(const Format& fmt) {
     demod_scale = (float)(fs / (2.0 * kPi));
     d0 = fmt.ire0 * 2.0 * kPi / fs;
     const float d0f = (float)d0;
+    {
+      const float pi = 3.14159265358979f;
+      auto wraps = [&](float r) {
+        volatile float sum = r + d0f;  // rounded to FP32
+        return sum > pi;
+      };
+      wrap = pi - d0f;
+      while (wraps(wrap)) wrap = std::nextafterf(wrap, -4.0f);
+      while (!wraps(std::nextafterf(wrap, 4.0f))) wrap = std::nextafterf(wrap, 4.0f);
+    }
     rot_re = (float)std::cos((double)d0f);
     rot_im = (float)-std::sin((double)d0f);
     demod_offset = (float)((double)d0f * (fs / (2.0 * kPi)) - fmt.ire0);

@@ -21,6 +21,9 @@ namespace {
 
 constexpr int kThreadsA = Design::kNa / 16;
 constexpr int kThreadsB = Design::kNb / 16;
+// K1a: the exchange buffer and half a spectrum; K1b: two exchange buffers
+constexpr size_t kSmemA = sizeof(float2) * (fft_pad(Design::kNa) + Design::kNa / 2);
+constexpr size_t kSmemB = 2 * sizeof(float2) * fft_pad(Design::kNb);
 
 __device__ __forceinline__ int wrap_tile(int q, int tile) {
   return q < 0 ? q + tile : (q >= tile ? q - tile : q);
@@ -31,44 +34,14 @@ __device__ __forceinline__ int wrap_tile(int q, int tile) {
 // u = x1 + i*x2.  With m = -k mod N, X1[k] = (U[k] + conj(U[m]))/2 and
 // X2[k] = (U[k] - conj(U[m]))/2i, so Z1 = X1*g and Z2 = X2*g follow from U and
 // its mirror (g is stored halved); each is inverted on its own.  Three
-// transforms serve two blocks instead of four.  ONE_SIDED (the analytic-signal
-// kernel of K1a, whose tile response is zero at negative frequencies) skips
-// bins k >= N/2: they are not formed and enter the inverse as zeros, which
-// also prunes the inverse's first pass.
+// transforms serve two blocks instead of four.  The analytic-signal kernel of
+// K1a has no negative frequencies: its bins k >= N/2 are not formed and the
+// inverse's first pass is that of a half-empty input.
 //
-// On return v holds Z1 (RegFFT layout) and sA holds Z2 in natural order; sB
-// is free once the caller's next barrier has passed.
-template <int N, bool ONE_SIDED>
-__device__ __forceinline__ void pair_spectra(float2 (&v)[16], float2* sA, float2* sB, const float2* __restrict__ g,
-                                             const float2* __restrict__ tw, int t) {
-  constexpr int T = N / 16;
-  RegFFT<N>::template run<false>(v, sA, tw, t);
-#pragma unroll
-  for (int q = 0; q < 16; q++) sB[pidx(t + T * q)] = v[q];
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 16; q++) {
-    if (ONE_SIDED && q >= 8) {
-      v[q] = make_float2(0.0f, 0.0f);  // k >= N/2: the kernel passes no negative frequencies
-      continue;
-    }
-    const int k = t + T * q;
-    const float2 um = sB[pidx((N - k) & (N - 1))];
-    const float2 u = v[q];
-    const float2 gg = __ldg(&g[k]);
-    const float2 x1 = make_float2(u.x + um.x, u.y - um.y);
-    const float2 x2 = make_float2(u.y + um.y, um.x - u.x);
-    v[q] = make_float2(x1.x * gg.x - x1.y * gg.y, x1.x * gg.y + x1.y * gg.x);
-    sA[pidx(k)] = make_float2(x2.x * gg.x - x2.y * gg.y, x2.x * gg.y + x2.y * gg.x);
-  }
-}
-
-// Z2 back from sA into the RegFFT layout (slots q >= 8 are zero when ONE_SIDED).
-template <int N, bool ONE_SIDED>
-__device__ __forceinline__ void load_second(float2 (&v)[16], const float2* sA, int t) {
-  constexpr int T = N / 16;
-#pragma unroll
-  for (int q = 0; q < 16; q++) v[q] = (ONE_SIDED && q >= 8) ? make_float2(0.0f, 0.0f) : sA[pidx(t + T * q)];
+// Bin k of both blocks: u = U[k], um = U[m], g = g[k].
+__device__ __forceinline__ void split_bin(float2 u, float2 um, float2 g, float2& z1, float2& z2) {
+  z1 = cmul_tw<false>(make_float2(u.x + um.x, u.y - um.y), g);
+  z2 = cmul_tw<false>(make_float2(u.y + um.y, um.x - u.x), g);
 }
 
 // Angle of (x, y) in [-pi, pi], the phase step of K1a: octant reduction to
@@ -77,90 +50,165 @@ __device__ __forceinline__ void load_second(float2 (&v)[16], const float2* sA, i
 // reweighted to minimax on [0, 1]; within 1.7 ulp of atan in FP32), and the
 // octant restored.  About half the instructions of a library atan2 and within
 // a few FP32 ulp of the angle: a few hundredths of a hertz of demodulated
-// frequency, below the FP32 rounding of the stage.
-__device__ __forceinline__ float phase_angle(float y, float x) {
-  const float ax = fabsf(x), ay = fabsf(y);
-  const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
-  const float t = mx > 0.0f ? __fdividef(mn, mx) : 0.0f;
-  const float s = t * t;
-  float q = 0.00262222f;
-  q = fmaf(q, s, -0.01513242f);
-  q = fmaf(q, s, 0.04112168f);
-  q = fmaf(q, s, -0.07366692f);
-  q = fmaf(q, s, 0.10573926f);
-  q = fmaf(q, s, -0.14185974f);
-  q = fmaf(q, s, 0.19990396f);
-  q = fmaf(q, s, -0.33332986f);
-  float r = fmaf(t * s, q, t);
-  if (ay > ax) r = 1.57079632679489662f - r;
-  if (x < 0.0f) r = 3.14159265358979324f - r;
-  return copysignf(r, y);
+// frequency, below the FP32 rounding of the stage.  Two angles at a time, the
+// polynomial packed and everything branch-free, so that the work of several
+// samples interleaves.
+__device__ __forceinline__ float angle_ratio(float2 c) {
+  const float ax = fabsf(c.x), ay = fabsf(c.y);
+  float inv;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(fmaxf(ax, ay)));
+  // 0/0 gives NaN, which fmaxf turns into the angle 0
+  return fmaxf(fminf(ax, ay) * inv, 0.0f);
+}
+__device__ __forceinline__ float angle_octant(float r, float2 c) {
+  if (fabsf(c.y) > fabsf(c.x)) r = 1.57079632679489662f - r;
+  if (c.x < 0.0f) r = 3.14159265358979324f - r;
+  return copysignf(r, c.y);
+}
+// Angles of the complex values a and b.
+__device__ __forceinline__ float2 phase_angle2(float2 a, float2 b) {
+  const F2 t = f2(angle_ratio(a), angle_ratio(b));
+  const F2 s = t * t;
+  F2 q = f2(0.00262222f, 0.00262222f);
+  q = f2_fma(q, s, f2(-0.01513242f, -0.01513242f));
+  q = f2_fma(q, s, f2(0.04112168f, 0.04112168f));
+  q = f2_fma(q, s, f2(-0.07366692f, -0.07366692f));
+  q = f2_fma(q, s, f2(0.10573926f, 0.10573926f));
+  q = f2_fma(q, s, f2(-0.14185974f, -0.14185974f));
+  q = f2_fma(q, s, f2(0.19990396f, 0.19990396f));
+  q = f2_fma(q, s, f2(-0.33332986f, -0.33332986f));
+  const float2 r = parts(f2_fma(t * s, q, t));
+  return make_float2(angle_octant(r.x, a), angle_octant(r.y, b));
+}
+
+// Square roots of two powers, correctly rounded for the finite normal values
+// a power takes (0 stays 0): the reciprocal square root estimate, one Newton
+// step, and a correction by the exact residual (P. Markstein, IBM J. Res.
+// Dev. 34, 1990).  Without the branch that a general square root takes for
+// subnormal values, which kept the work of successive samples apart.
+__device__ __forceinline__ float2 root2(float a, float b) {
+  float ya, yb;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(a));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
+  const F2 x = f2(a, b), y = f2(ya, yb), g = x * y;
+  const float2 gp = parts(g);
+  const float2 s = parts(f2_fma(f2_fma(f2(-gp.x, -gp.y), g, x), y * f2(0.5f, 0.5f), g));
+  return make_float2(fmaxf(s.x, 0.0f), fmaxf(s.y, 0.0f));
+}
+
+// Predicated accesses: two words to global memory, a complex value from shared
+// memory.  (Written as an if, each became a branch of its own.)
+__device__ __forceinline__ void st_global_if(bool on, float* p, float x, float* q, float y) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p st.global.f32 [%1], %2;\n\t@p st.global.f32 [%3], %4;\n\t}" ::"r"(
+          (int)on),
+      "l"(p), "f"(x), "l"(q), "f"(y)
+      : "memory");
+}
+__device__ __forceinline__ void ld_shared_if(int on, float2& v, uint32_t addr) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p ld.shared.v2.f32 {%0, %1}, [%3];\n\t}"
+               : "+f"(v.x), "+f"(v.y)
+               : "r"(on), "r"(addr)
+               : "memory");
 }
 
 // K1a output stage for one block: phase step (FP32 Hz, relative to ire0) and
 // envelope of outputs [j0, j0 + nout) of tile f, and the block's envelope sum.
 // z (thread t, slot q) is block sample t + T*q; its predecessor is held by
 // thread t-1 (same q), or for t = 0 by thread T-1 at q-1.
+//
+// Half of the kernel's instructions are here (64 an output with one sample at
+// a time behind a range test).  Slots are taken two at a time in packed
+// arithmetic, every slot computed and only the stores tested, so that the
+// compiler interleaves them; the outermost slots, mostly or wholly outside
+// the outputs, are paired with each other and skipped where both lie outside.
 template <int T>
 __device__ __forceinline__ void k1a_emit(const DemodArgs& a, const float2 (&z)[16], int f, int j0, int block,
-                                         float2 (*warp_last)[16], double* red, int t) {
+                                         float2 (*warp_last)[18], double* red, int t) {
   const int lane = t & 31, warp = t >> 5;
+  constexpr int W = T / 32;
+  // row w of warp_last: the predecessors of warp w's first lane, slot q
   if (lane == 31) {
+    float2* row = warp < W - 1 ? warp_last[warp + 1] : warp_last[0] + 1;
 #pragma unroll
-    for (int q = 0; q < 16; q++) warp_last[warp][q] = z[q];
+    for (int q = 0; q < 16; q++) row[q] = z[q];
   }
   __syncthreads();
   const int nout = min(a.a_out, kOverlap + a.spp - j0);
-  float* dem_out = a.dem + (f * a.spp + (j0 - kOverlap));
-  float* env_out = a.env + (f * a.spp + (j0 - kOverlap));
-  double esum = 0.0;
-#pragma unroll
-  for (int q = 0; q < 16; q++) {
+  const int i0 = t - (a.a_pos + 1);  // output index of slot 0
+  float* dem_out = a.dem + (f * a.spp + (j0 - kOverlap)) + i0;
+  float* env_out = a.env + (f * a.spp + (j0 - kOverlap)) + i0;
+  const F2 rot = f2(a.rot_re, a.rot_im), rot_q = f2(-a.rot_im, a.rot_re);
+  float e[16];
+  const int first = lane == 0;
+  const uint32_t prev = (uint32_t)__cvta_generic_to_shared(warp_last[warp]);
+  // the step of slot q: z * conj(zp) rotated by the nominal step, so the angle is small
+  auto step = [&](int q) {
     float2 zp;
     zp.x = __shfl_up_sync(0xffffffffu, z[q].x, 1);
     zp.y = __shfl_up_sync(0xffffffffu, z[q].y, 1);
-    if (lane == 0) zp = warp > 0 ? warp_last[warp - 1][q] : (q > 0 ? warp_last[T / 32 - 1][q - 1] : z[q]);
-    const int i = t + T * q - (a.a_pos + 1);
-    if (i >= 0 && i < nout) {
-      const float2 zz = z[q];
-      // z * conj(zp) rotated by the nominal step, so atan2 sees a small angle
-      const float re0 = zz.x * zp.x + zz.y * zp.y;
-      const float im0 = zz.y * zp.x - zz.x * zp.y;
-      const float re = re0 * a.rot_re - im0 * a.rot_im;
-      const float im = re0 * a.rot_im + im0 * a.rot_re;
-      float r = phase_angle(im, re);
-      // keep the un-rotated step in (-pi, pi] as the reference's wrap does
-      if (r + a.d0 > 3.14159265358979f) r -= 6.28318530717959f;
-      dem_out[i] = r * a.demod_scale + a.demod_offset;
-      const float e = sqrtf(zz.x * zz.x + zz.y * zz.y);
-      env_out[i] = e;
-      esum += (double)e;
-    }
+    ld_shared_if(first, zp, prev + 8 * q);
+    const float2 zz = z[q];
+    const float2 c = parts(f2_fma(f2(zz), f2(zp.x, zp.x), f2(zz.y, zz.x) * f2(zp.y, -zp.y)));
+    return parts(f2_fma(f2(c.x, c.x), rot, f2(c.y, c.y) * rot_q));
+  };
+  auto power = [](float2 v) { return fmaf(v.x, v.x, v.y * v.y); };
+  auto emit = [&](int qa, int qb) {
+    float2 r = phase_angle2(step(qa), step(qb));
+    // keep the un-rotated step in (-pi, pi] as the reference's wrap does
+    if (r.x > a.wrap) r.x -= 6.28318530717959f;
+    if (r.y > a.wrap) r.y -= 6.28318530717959f;
+    const float2 hz = parts(f2_fma(f2(r), f2(a.demod_scale, a.demod_scale), f2(a.demod_offset, a.demod_offset)));
+    const float2 m = root2(power(z[qa]), power(z[qb]));
+    e[qa] = m.x;
+    e[qb] = m.y;
+    st_global_if((unsigned)(i0 + T * qa) < (unsigned)nout, dem_out + T * qa, hz.x, env_out + T * qa, m.x);
+    st_global_if((unsigned)(i0 + T * qb) < (unsigned)nout, dem_out + T * qb, hz.y, env_out + T * qb, m.y);
+  };
+  const int lead = a.a_pos + 1;
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    e[p] = e[15 - p] = 0.0f;
+    if (T * p + T - 1 >= lead || T * (15 - p) - lead < nout) emit(p, 15 - p);
   }
+#pragma unroll
+  for (int q = 2; q < 14; q += 2) emit(q, q + 1);
   // Deterministic per-block envelope partial sums (the dropout stage needs
   // the tile mean).
+  double esum = 0.0;
+#pragma unroll
+  for (int q = 0; q < 16; q++)
+    if ((unsigned)(i0 + T * q) < (unsigned)nout) esum += (double)e[q];
   for (int off = 16; off > 0; off >>= 1) esum += __shfl_down_sync(0xffffffffu, esum, off);
   if (lane == 0) red[warp] = esum;
   __syncthreads();
   if (t == 0) {
     double sacc = 0.0;
-    for (int w = 0; w < T / 32; w++) sacc += red[w];
+    for (int w = 0; w < W; w++) sacc += red[w];
     a.env_part[(size_t)f * a.env_blocks + block] = sacc;
   }
 }
 
 // K1a: u8 -> analytic signal -> phase step + envelope, blocks 2x and 2x+1 of
 // the tile (the second may lie past the tile's end).
+//
+// Bound by an SM's units side by side, none of them full: FP32 pipe 49%, shared
+// memory 46%, load/store 41%, issue 57% of cycles; DRAM 9%.  64 registers and
+// 51 KB of shared memory put four CTAs on an SM, in different parts of their
+// transforms (three at 80 registers: 130 us).  The second block's half
+// spectrum waits in shared memory, and U is exchanged in the transform's own
+// buffer.  40 fields at 28 MHz: 171 -> 126 us, 168 MB of interface traffic at
+// 984 -> 1,335 GB/s.  (Two pairs of blocks in the two lanes of packed
+// arithmetic, four blocks a CTA at 128 registers and two CTAs an SM: 187 us.)
 template <int FMT, class Src>
-__global__ void __launch_bounds__(kThreadsA, 3) k1a_kernel(const __grid_constant__ Src src, int f_begin) {
+__global__ void __launch_bounds__(kThreadsA, 4) k1a_kernel(const __grid_constant__ Src src, int f_begin) {
   constexpr int N = Design::kNa, T = kThreadsA;
   const DemodArgs& a = src.get();
   if (f_begin + (int)blockIdx.y >= a.tiles) return;  // whole CTA: a batched capture with fewer tiles
   chain_wait();
   extern __shared__ float2 sm[];
-  float2* sA = sm;
-  float2* sB = sm + fft_pad(N);
-  __shared__ float2 warp_last[T / 32][16];
+  float2* z2 = sm + fft_pad(N);  // the second block's spectrum, each slot its own thread's
+  __shared__ float2 warp_last[T / 32][18];
   __shared__ double red[T / 32];
   const int t = threadIdx.x;
   const int f = f_begin + blockIdx.y;
@@ -177,10 +225,12 @@ __global__ void __launch_bounds__(kThreadsA, 3) k1a_kernel(const __grid_constant
   const float dc = a.dc ? *a.dc : 0.0f;
   if (base >= 0 && base + span <= a.tile && tile0 + base >= 0 && tile0 + base + span - 1 <= last &&
       tile0 + base + span <= a.n_read) {
-    const int p = tile0 + base + t;
+    // one address a block, constant offsets from it
+    const uint8_t* p0 = raw_at<FMT>(a.raw, tile0 + base + t);
+    const uint8_t* p1 = raw_at<FMT>(p0, a.a_out);
 #pragma unroll
     for (int q = 0; q < 16; q++)
-      v[q] = make_float2(raw_convert<FMT>(a.raw, p + T * q) - dc, raw_convert<FMT>(a.raw, p + T * q + a.a_out) - dc);
+      v[q] = make_float2(raw_convert<FMT>(p0, T * q) - dc, raw_convert<FMT>(p1, T * q) - dc);
   } else {
 #pragma unroll
     for (int q = 0; q < 16; q++) {
@@ -190,18 +240,59 @@ __global__ void __launch_bounds__(kThreadsA, 3) k1a_kernel(const __grid_constant
       v[q] = make_float2(raw_sample<FMT>(a.raw, p0, a.n_read, dc), raw_sample<FMT>(a.raw, p1, a.n_read, dc));
     }
   }
-  pair_spectra<N, true>(v, sA, sB, a.ga, a.tw_a, t);
+  RegFFT<N>::run<false>(v, sm, a.tw_a, t);
+  __syncthreads();  // the last pass's reads
+#pragma unroll
+  for (int q = 0; q < 16; q++) sm[pidx(t + T * q)] = v[q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const int k = t + T * q;
+    split_bin(v[q], sm[pidx((N - k) & (N - 1))], __ldg(&a.ga[k]), v[q], z2[k]);
+  }
   // one copy of the inverse transform and output stage serves both blocks
   // (a rolled loop keeps the kernel body small for the instruction cache)
 #pragma unroll 1
   for (int b = 0; b < 2; b++) {
     if (b == 1) {
       if (blk0 + 1 >= a.env_blocks) return;  // whole CTA
-      load_second<N, true>(v, sA, t);
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = z2[t + T * q];
     }
-    RegFFT<N>::run<true>(v, b == 0 ? sB : sA, a.tw_a_inv, t);
+    RegFFT<N>::run_half<true>(v, sm, a.tw_a_inv, t);
     k1a_emit<T>(a, v, f, j0 + b * a.a_out, blk0 + b, warp_last, red, t);
   }
+}
+
+// On return v holds Z1 (RegFFT layout) and sA holds Z2 in natural order; sB
+// is free once the caller's next barrier has passed.
+template <int N>
+__device__ __forceinline__ void pair_spectra(float2 (&v)[16], float2* sA, float2* sB, const float2* __restrict__ g,
+                                             const float2* __restrict__ tw, int t) {
+  constexpr int T = N / 16;
+  RegFFT<N>::template run<false>(v, sA, tw, t);
+#pragma unroll
+  for (int q = 0; q < 16; q++) sB[pidx(t + T * q)] = v[q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int k = t + T * q;
+    const float2 um = sB[pidx((N - k) & (N - 1))];
+    const float2 u = v[q];
+    const float2 gg = __ldg(&g[k]);
+    const float2 x1 = make_float2(u.x + um.x, u.y - um.y);
+    const float2 x2 = make_float2(u.y + um.y, um.x - u.x);
+    v[q] = make_float2(x1.x * gg.x - x1.y * gg.y, x1.x * gg.y + x1.y * gg.x);
+    sA[pidx(k)] = make_float2(x2.x * gg.x - x2.y * gg.y, x2.x * gg.y + x2.y * gg.x);
+  }
+}
+
+// Z2 back from sA into the RegFFT layout.
+template <int N>
+__device__ __forceinline__ void load_second(float2 (&v)[16], const float2* sA, int t) {
+  constexpr int T = N / 16;
+#pragma unroll
+  for (int q = 0; q < 16; q++) v[q] = sA[pidx(t + T * q)];
 }
 
 // K1b output stage: video (real part) and sync (imaginary part) of one block.
@@ -283,11 +374,11 @@ __global__ void __launch_bounds__(kThreadsB, 1) k1b_kernel(const __grid_constant
       v[q] = make_float2(__ldg(&a.dem[p0]), __ldg(&a.dem[p1]));
     }
   }
-  pair_spectra<N, false>(v, sA, sB, a.gb, a.tw_b, t);
+  pair_spectra<N>(v, sA, sB, a.gb, a.tw_b, t);
   // both blocks' inverses in lockstep (sB and sA as their buffers)
   float2 v2[16];
   __syncthreads();  // Z2 complete in sA
-  load_second<N, false>(v2, sA, t);
+  load_second<N>(v2, sA, t);
   RegFFT<N>::run2<true>(v, sB, v2, sA, a.tw_b_inv, opaque_index(t));
   k1b_emit<T>(a, v, f, j0, t);
   if (kOverlap + (blk0 + 1) * a.b_out >= kOverlap + a.spp) return;  // the second block lies past the tile
@@ -565,7 +656,7 @@ void launch_edges_bits_many(const ArgsMany<EdgeArgs>& e, int portions, long long
 
 void launch_k1a(const DemodArgs& a, int f0, int nf, cudaStream_t st) {
   if (nf <= 0) return;
-  const size_t smem = 2 * sizeof(float2) * fft_pad(Design::kNa);
+  const size_t smem = kSmemA;
   const int blocks = (a.spp + a.a_out - 1) / a.a_out;  // = env_blocks
   dim3 grid((blocks + 1) / 2, nf);
   const ArgsOne<DemodArgs> src{a};
@@ -582,7 +673,7 @@ void launch_k1a(const DemodArgs& a, int f0, int nf, cudaStream_t st) {
 void launch_k1a_many(const ArgsMany<DemodArgs>& p, int portions, int max_tiles, cudaStream_t st) {
   if (portions <= 0 || max_tiles <= 0) return;
   const DemodArgs& a = p.a[0];  // the design constants every capture of a round shares
-  const size_t smem = 2 * sizeof(float2) * fft_pad(Design::kNa);
+  const size_t smem = kSmemA;
   const int blocks = (a.spp + a.a_out - 1) / a.a_out;
   dim3 grid((blocks + 1) / 2, max_tiles, portions);
   auto go = [&](auto kernel) {
@@ -634,7 +725,7 @@ void launch_dc_mean(const uint8_t* raw, int n, int in_fmt, unsigned long long* s
 
 void launch_k1b(const DemodArgs& a, int f0, int nf, cudaStream_t st) {
   if (nf <= 0) return;
-  const size_t smem = 2 * sizeof(float2) * fft_pad(Design::kNb);
+  const size_t smem = kSmemB;
   using S = ArgsOne<DemodArgs>;
   cudaFuncSetAttribute(k1b_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int blocks = (a.spp + a.b_out - 1) / a.b_out;
@@ -646,7 +737,7 @@ void launch_k1b(const DemodArgs& a, int f0, int nf, cudaStream_t st) {
 void launch_k1b_many(const ArgsMany<DemodArgs>& p, int portions, int max_tiles, cudaStream_t st) {
   if (portions <= 0 || max_tiles <= 0) return;
   const DemodArgs& a = p.a[0];
-  const size_t smem = 2 * sizeof(float2) * fft_pad(Design::kNb);
+  const size_t smem = kSmemB;
   using S = ArgsMany<DemodArgs>;
   cudaFuncSetAttribute(k1b_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int blocks = (a.spp + a.b_out - 1) / a.b_out;

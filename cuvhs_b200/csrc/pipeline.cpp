@@ -602,7 +602,7 @@ DemodArgs Context::demod_args(int T) const {
   da.b_out = des.b_out;
   da.rot_re = des.rot_re;
   da.rot_im = des.rot_im;
-  da.d0 = (float)des.d0;
+  da.wrap = des.wrap;
   da.demod_scale = des.demod_scale;
   da.demod_offset = des.demod_offset;
   da.corr_video = des.corr_video;

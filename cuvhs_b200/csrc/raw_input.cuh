@@ -22,6 +22,12 @@ __device__ __forceinline__ float raw_convert(const uint8_t* __restrict__ raw, in
   return (float)__ldg(reinterpret_cast<const uint16_t*>(raw) + p) - 32768.0f;
 }
 
+// Address of sample p (raw_convert<FMT> at an index from it).
+template <int FMT>
+__device__ __forceinline__ const uint8_t* raw_at(const uint8_t* raw, int p) {
+  return raw + (long long)p * (FMT == kInU8 ? 1 : 2);
+}
+
 // Sample p of the chunk: converted, DC removed, 0 past the samples read.
 template <int FMT>
 __device__ __forceinline__ float raw_sample(const uint8_t* __restrict__ raw, int p, int n_read, float dc) {
