@@ -15,15 +15,18 @@
 #include "cuvhs_internal.h"
 #include "raw_input.cuh"
 #include "reg_fft.cuh"
+#include "tmem.cuh"
 
 namespace cuvhs {
 namespace {
 
 constexpr int kThreadsA = Design::kNa / 16;
 constexpr int kThreadsB = Design::kNb / 16;
-// K1a: the exchange buffer and half a spectrum; K1b: two exchange buffers
+// K1a: the exchange buffer and half a spectrum; K1b: the exchange buffer, with
+// a spectrum of 32 words a thread in tensor memory
 constexpr size_t kSmemA = sizeof(float2) * (fft_pad(Design::kNa) + Design::kNa / 2);
-constexpr size_t kSmemB = 2 * sizeof(float2) * fft_pad(Design::kNb);
+constexpr size_t kSmemB = sizeof(float2) * fft_pad(Design::kNb);
+constexpr int kTmemColsB = 32 * (kThreadsB / 128);
 
 __device__ __forceinline__ int wrap_tile(int q, int tile) {
   return q < 0 ? q + tile : (q >= tile ? q - tile : q);
@@ -264,44 +267,15 @@ __global__ void __launch_bounds__(kThreadsA, 4) k1a_kernel(const __grid_constant
   }
 }
 
-// On return v holds Z1 (RegFFT layout) and sA holds Z2 in natural order; sB
-// is free once the caller's next barrier has passed.
-template <int N>
-__device__ __forceinline__ void pair_spectra(float2 (&v)[16], float2* sA, float2* sB, const float2* __restrict__ g,
-                                             const float2* __restrict__ tw, int t) {
-  constexpr int T = N / 16;
-  RegFFT<N>::template run<false>(v, sA, tw, t);
-#pragma unroll
-  for (int q = 0; q < 16; q++) sB[pidx(t + T * q)] = v[q];
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 16; q++) {
-    const int k = t + T * q;
-    const float2 um = sB[pidx((N - k) & (N - 1))];
-    const float2 u = v[q];
-    const float2 gg = __ldg(&g[k]);
-    const float2 x1 = make_float2(u.x + um.x, u.y - um.y);
-    const float2 x2 = make_float2(u.y + um.y, um.x - u.x);
-    v[q] = make_float2(x1.x * gg.x - x1.y * gg.y, x1.x * gg.y + x1.y * gg.x);
-    sA[pidx(k)] = make_float2(x2.x * gg.x - x2.y * gg.y, x2.x * gg.y + x2.y * gg.x);
-  }
-}
-
-// Z2 back from sA into the RegFFT layout.
-template <int N>
-__device__ __forceinline__ void load_second(float2 (&v)[16], const float2* sA, int t) {
-  constexpr int T = N / 16;
-#pragma unroll
-  for (int q = 0; q < 16; q++) v[q] = sA[pidx(t + T * q)];
-}
-
 // K1b output stage: video (real part) and sync (imaginary part) of one block.
 // Sync samples within guard_hz of the pulse threshold are listed for the FP64
-// re-evaluation (kernels_guard.cu); a handful per field.
+// re-evaluation (kernels_guard.cu); a handful per field, so the slot loop only
+// notes that there is one.
 template <int T>
 __device__ __forceinline__ void k1b_emit(const DemodArgs& a, const float2 (&z)[16], int f, int j0, int t) {
   const int nout = min(a.b_out, kOverlap + a.spp - j0);
-  const int out0 = f * a.spp + (j0 - kOverlap);
+  const int i0 = t - a.b_pos;                        // output index of slot 0
+  const int out0 = f * a.spp + (j0 - kOverlap) + i0;  // its chunk position
   float* video_out = a.video + out0;
   float* sync_out = a.sync + out0;
   const int lane = t & 31;
@@ -309,27 +283,31 @@ __device__ __forceinline__ void k1b_emit(const DemodArgs& a, const float2 (&z)[1
   // lane q keeps slot q's ballot, and after the loop lanes 0..15 OR their
   // words into the (at most two) bit words each straddles, in parallel
   unsigned mine = 0;
+  bool near = false;
+  const F2 corr = f2(a.corr_video, a.corr_sync);
 #pragma unroll
   for (int q = 0; q < 16; q++) {
-    const int i = t + T * q - a.b_pos;
-    bool in = false;
-    if (i >= 0 && i < nout) {
-      video_out[i] = z[q].x + a.corr_video;
-      const float sv = z[q].y + a.corr_sync;
-      sync_out[i] = sv;
-      in = sv <= a.thr_rel;
-      if (fabsf(sv - a.thr_rel) < a.guard_hz && a.guard_list) {
-        const int slot = atomicAdd(a.guard_count, 1);
-        if (slot < a.guard_cap) {
-          a.guard_list[slot] = (unsigned)(out0 + i);
-        }
-      }
+    const float2 o = parts(f2(z[q]) + corr);
+    const bool valid = (unsigned)(i0 + T * q) < (unsigned)nout;
+    if (valid) {
+      video_out[T * q] = o.x;
+      sync_out[T * q] = o.y;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, in);
+    near = near || (valid && fabsf(o.y - a.thr_rel) < a.guard_hz);
+    const unsigned m = __ballot_sync(0xffffffffu, valid && o.y <= a.thr_rel);
     mine = lane == q ? m : mine;
   }
+  if (__any_sync(0xffffffffu, near) && a.guard_list) {
+#pragma unroll 1
+    for (int q = 0; q < 16; q++) {
+      if ((unsigned)(i0 + T * q) < (unsigned)nout && fabsf(sync_out[T * q] - a.thr_rel) < a.guard_hz) {
+        const int slot = atomicAdd(a.guard_count, 1);
+        if (slot < a.guard_cap) a.guard_list[slot] = (unsigned)(out0 + T * q);
+      }
+    }
+  }
   if (a.pulse_bits && mine) {  // only lanes 0..15 hold a word
-    long long p0 = (long long)out0 + (t - lane) + (long long)T * lane - a.b_pos;
+    long long p0 = (long long)(out0 - lane) + (long long)T * lane;
     if (p0 < 0) {  // positions before the chunk start hold no bits
       mine >>= (int)(-p0);
       p0 = 0;
@@ -342,16 +320,25 @@ __device__ __forceinline__ void k1b_emit(const DemodArgs& a, const float2 (&z)[1
 }
 
 // K1b: demod -> video + sync, blocks 2x and 2x+1 of the tile.
+//
+// One 8192-point exchange buffer (70 KB) and 64 registers a thread put two
+// CTAs on an SM, one's arithmetic beside the other's exchanges: the second
+// block's spectrum (64 KB, which shared memory does not hold twice more) waits
+// in tensor memory, each thread's 32 words in columns of its own.  Both
+// inverses in lockstep at 128 registers and one CTA an SM left every unit
+// below 38% (issue 44%); now FP32 pipe 41%, shared memory 44%, load/store 37%,
+// issue 52%, DRAM 17%.  40 fields at 28 MHz: 179 -> 140 us, 227 MB of
+// interface traffic at 1,266 -> 1,618 GB/s.
 template <class Src>
-__global__ void __launch_bounds__(kThreadsB, 1) k1b_kernel(const __grid_constant__ Src src, int f_begin) {
+__global__ void __launch_bounds__(kThreadsB, 2) k1b_kernel(const __grid_constant__ Src src, int f_begin) {
   constexpr int N = Design::kNb, T = kThreadsB;
   const DemodArgs& a = src.get();
   if (f_begin + (int)blockIdx.y >= a.tiles) return;  // whole CTA
-  chain_wait();
   extern __shared__ float2 sm[];
-  float2* sA = sm;
-  float2* sB = sm + fft_pad(N);
-  const int t = threadIdx.x;
+  __shared__ uint32_t tmem_base;
+  const int t = threadIdx.x, warp = t >> 5;
+  tmem_alloc<kTmemColsB>(&tmem_base, warp);
+  chain_wait();
   const int f = f_begin + blockIdx.y;
   const int blk0 = 2 * blockIdx.x;
   const int j0 = kOverlap + blk0 * a.b_out;
@@ -362,9 +349,10 @@ __global__ void __launch_bounds__(kThreadsB, 1) k1b_kernel(const __grid_constant
   const int span = a.b_out + N;  // tile positions [base, base + span) are read
   if (base >= 0 && base + span <= a.tile && tile0 + base >= 0 && tile0 + base + span - 1 <= last) {
     // interior: no wrap inside the tile, no clamp at the chunk ends
-    const float* p = a.dem + (tile0 + base + t);
+    const float* p0 = a.dem + (tile0 + base + t);
+    const float* p1 = p0 + a.b_out;
 #pragma unroll
-    for (int q = 0; q < 16; q++) v[q] = make_float2(__ldg(p + T * q), __ldg(p + T * q + a.b_out));
+    for (int q = 0; q < 16; q++) v[q] = make_float2(__ldg(p0 + T * q), __ldg(p1 + T * q));
   } else {
 #pragma unroll
     for (int q = 0; q < 16; q++) {
@@ -374,15 +362,39 @@ __global__ void __launch_bounds__(kThreadsB, 1) k1b_kernel(const __grid_constant
       v[q] = make_float2(__ldg(&a.dem[p0]), __ldg(&a.dem[p1]));
     }
   }
-  pair_spectra<N>(v, sA, sB, a.gb, a.tw_b, t);
-  // both blocks' inverses in lockstep (sB and sA as their buffers)
-  float2 v2[16];
-  __syncthreads();  // Z2 complete in sA
-  load_second<N>(v2, sA, t);
-  RegFFT<N>::run2<true>(v, sB, v2, sA, a.tw_b_inv, opaque_index(t));
-  k1b_emit<T>(a, v, f, j0, t);
-  if (kOverlap + (blk0 + 1) * a.b_out >= kOverlap + a.spp) return;  // the second block lies past the tile
-  k1b_emit<T>(a, v2, f, j0 + a.b_out, t);
+  RegFFT<N>::run<false>(v, sm, a.tw_b, t);
+  __syncthreads();  // the last pass's reads
+#pragma unroll
+  for (int q = 0; q < 16; q++) sm[pidx(t + T * q)] = v[q];
+  __syncthreads();
+  // the second block's spectrum waits in tensor memory
+  const uint32_t own = tmem_own(tmem_base, warp, 32);
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    float2 z2[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int q = 4 * c + i, k = t + T * q;
+      split_bin(v[q], sm[pidx((N - k) & (N - 1))], __ldg(&a.gb[k]), v[q], z2[i]);
+    }
+    tmem_st8(own + 8 * c, z2);
+  }
+  tmem_wait_st();
+  // one copy of the inverse transform and output stage serves both blocks
+  const int nblk = kOverlap + (blk0 + 1) * a.b_out >= kOverlap + a.spp ? 1 : 2;  // the second may lie past the tile
+#pragma unroll 1
+  for (int b = 0; b < nblk; b++) {
+    if (b == 1) {
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 4; c++) tmem_ld8(own + 8 * c, v + 4 * c);
+      tmem_wait_ld();
+    }
+    RegFFT<N>::run<true>(v, sm, a.tw_b_inv, opaque_index(t));
+    k1b_emit<T>(a, v, f, j0 + b * a.b_out, t);
+  }
+  __syncthreads();
+  tmem_free<kTmemColsB>(tmem_base, warp);
 }
 
 // Threshold edges in sample order.  Each thread owns 16 consecutive samples

@@ -90,77 +90,6 @@ struct RegFFT {
     if constexpr (!LAST) rest<NS * fft_radix(N, NS), INV>(v, s, tw, t);
   }
 
-  // Two independent transforms of the same direction in lockstep: v1 with
-  // buffer s1, v2 with buffer s2.  Each pass loads a twiddle once for both,
-  // waits on one barrier for both, and has twice the independent arithmetic;
-  // every value is computed exactly as by two run() calls.
-  template <int NS, bool INV, bool LAST>
-  __device__ __forceinline__ static void pass2(float2 (&v1)[16], float2* s1, float2 (&v2)[16], float2* s2,
-                                               const float2* __restrict__ tw, int t) {
-    constexpr int R = fft_radix(N, NS);
-    constexpr int B = 16 / R;
-    static_assert(LAST || B == 1, "only the last pass has a smaller radix");
-    const int at = place<NS>(t);
-    float2 w1[B][R], w2[B][R];
-#pragma unroll
-    for (int b = 0; b < B; b++) {
-      const int k = (t + T * b) & (NS - 1);
-      const float2* twp = tw + (NS - 16) + k;
-      const int o = at + b * butterfly_stride<NS>();
-      w1[b][0] = s1[o];
-      w2[b][0] = s2[o];
-#pragma unroll
-      for (int r = 1; r < R; r++) {
-        const float2 c = __ldg(&twp[(r - 1) * NS]);
-        w1[b][r] = cmul_tw<INV>(s1[o + r * slot_stride<NS>()], c);
-        w2[b][r] = cmul_tw<INV>(s2[o + r * slot_stride<NS>()], c);
-      }
-      dft<R, INV>(w1[b]);
-      dft<R, INV>(w2[b]);
-    }
-    if constexpr (LAST) {
-#pragma unroll
-      for (int b = 0; b < B; b++)
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          v1[b + B * r] = w1[b][dft_slot<R>(r)];
-          v2[b + B * r] = w2[b][dft_slot<R>(r)];
-        }
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        s1[at + r * slot_stride<NS>()] = w1[0][dft_slot<R>(r)];
-        s2[at + r * slot_stride<NS>()] = w2[0][dft_slot<R>(r)];
-      }
-      __syncthreads();
-    }
-  }
-
-  template <int NS, bool INV>
-  __device__ __forceinline__ static void rest2(float2 (&v1)[16], float2* s1, float2 (&v2)[16], float2* s2,
-                                               const float2* __restrict__ tw, int t) {
-    constexpr bool LAST = NS * fft_radix(N, NS) >= N;
-    pass2<NS, INV, LAST>(v1, s1, v2, s2, tw, t);
-    if constexpr (!LAST) rest2<NS * fft_radix(N, NS), INV>(v1, s1, v2, s2, tw, t);
-  }
-
-  // run() on two transforms at once (see pass2); s1 and s2 may be in use by
-  // the caller until this call.
-  template <bool INV>
-  __device__ __forceinline__ static void run2(float2 (&v1)[16], float2* s1, float2 (&v2)[16], float2* s2,
-                                              const float2* __restrict__ tw, int t) {
-    dft<16, INV>(v1);
-    dft<16, INV>(v2);
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 16; r++) {
-      s1[pidx(16 * t + r)] = v1[dft_slot<16>(r)];
-      s2[pidx(16 * t + r)] = v2[dft_slot<16>(r)];
-    }
-    __syncthreads();
-    rest2<16, INV>(v1, s1, v2, s2, tw, t);
-  }
-
   // Transform v in place.  The buffer s (fft_pad(N) float2) may be in use by
   // the caller until this call: the first write waits on a barrier.  On return
   // other threads may still be reading s: a barrier comes before its next use.
