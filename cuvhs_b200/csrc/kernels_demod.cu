@@ -386,9 +386,7 @@ __global__ void __launch_bounds__(kThreadsB, 2) k1b_kernel(const __grid_constant
   for (int b = 0; b < nblk; b++) {
     if (b == 1) {
       __syncwarp();
-#pragma unroll
-      for (int c = 0; c < 4; c++) tmem_ld8(own + 8 * c, v + 4 * c);
-      tmem_wait_ld();
+      tmem_ld32(own, v);
     }
     RegFFT<N>::run<true>(v, sm, a.tw_b_inv, opaque_index(t));
     k1b_emit<T>(a, v, f, j0 + b * a.b_out, t);
