@@ -11,6 +11,7 @@
 
 #include "adjoint.h"
 #include "reg_fft.cuh"
+#include "tmem.cuh"
 
 namespace cuvhs {
 namespace {
@@ -18,7 +19,6 @@ namespace {
 constexpr int kN = Design::kNb;
 constexpr int kT = kN / 16;
 constexpr int kRowThreads = 128;
-constexpr int kLineWarps = 4;
 // The calibration model is NTSC: 910-sample lines in a 1024-point line
 // transform, a 36-sample burst window.
 constexpr int kLineFFT = 1024;
@@ -79,10 +79,42 @@ __device__ __forceinline__ double row_start(const AdjArgs& a, int f, int r) {
   return a.ll[(size_t)f * a.lpf + r] + a.line_off[(size_t)f * (a.out_h + 1) + r];
 }
 
+// ----------------------------------------------------------------- filter
+__device__ __forceinline__ double2 zmul(double2 a, double2 b) {
+  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ double2 zdiv(double2 a, double2 b) {
+  const double q = b.x * b.x + b.y * b.y;
+  return make_double2((a.x * b.x + a.y * b.y) / q, (a.y * b.x - a.x * b.y) / q);
+}
+
+// A thread per bin.  Every call has new coefficients; building the spectra on
+// the host (8192 bins, five complex FP64 spectra with their exponentials) and
+// sending them took 0.5 ms of a 0.87 ms gradient; here they take 4 us.
+constexpr int kFilterThreads = 128;
+__global__ void __launch_bounds__(kFilterThreads) adj_filter_kernel(AdjFilterArgs a) {
+  const int k = blockIdx.x * kFilterThreads + threadIdx.x;
+  const double n0 = 1.0 + a.m1 + a.m2 - a.n1 - a.n2;
+  const double2 z1 = a.z1[k], z2 = zmul(z1, z1);
+  const double S = a.s[k] / kN;
+  const double2 num = make_double2(n0 + a.n1 * z1.x + a.n2 * z2.x, a.n1 * z1.y + a.n2 * z2.y);
+  const double2 den = make_double2(1.0 + a.m1 * z1.x + a.m2 * z2.x, a.m1 * z1.y + a.m2 * z2.y);
+  const double2 H = zdiv(num, den);
+  auto put = [&](float2* dst, double2 v) { dst[k] = make_float2((float)(v.x * S), (float)(v.y * S)); };
+  put(a.gv, H);
+  if (!a.dg) return;
+  // n0 moves with every coefficient
+  put(a.dg, zdiv(make_double2(z1.x - 1.0, z1.y), den));
+  put(a.dg + kN, zdiv(make_double2(z2.x - 1.0, z2.y), den));
+  const double2 h1 = zmul(H, z1), h2 = zmul(H, z2);
+  put(a.dg + 2 * kN, zdiv(make_double2(1.0 - h1.x, -h1.y), den));
+  put(a.dg + 3 * kN, zdiv(make_double2(1.0 - h2.x, -h2.y), den));
+}
+
 // ------------------------------------------------------------------ video
 // Overlap-save over [0, total) with zero padding; the kernel is real, so two
 // blocks ride in the real and imaginary parts of one transform.
-__global__ void __launch_bounds__(kT, 1) adj_video_kernel(AdjArgs a) {
+__global__ void __launch_bounds__(kT, 2) adj_video_kernel(AdjArgs a) {
   extern __shared__ float2 sm[];
   const int t = threadIdx.x;
   const long long j0 = (long long)(2 * blockIdx.x) * a.b_out;
@@ -187,42 +219,67 @@ __device__ __forceinline__ ChromaSample chroma_sample(const AdjArgs& a, int gl, 
   return o;
 }
 
+// A line pair is transformed by kPairThreads threads (two warps, synchronised
+// on their named barrier), kPairs pairs to a CTA.
+constexpr int kPairThreads = 64;
+constexpr int kPairs = 2;
+constexpr int kPerThread = kLineFFT / kPairThreads;  // columns a thread
+
 // 1024-point band-pass of the two lines held in sm (real and imaginary parts).
-__device__ __forceinline__ void line_bandpass(float2* sm, const AdjArgs& a, int lane) {
-  __syncwarp();
-  smem_fft<kLineFFT, 32, false>(sm, a.tw_l, lane);
+__device__ __forceinline__ void line_bandpass(float2* sm, const AdjArgs& a, int tid) {
+  fft_sync<kPairThreads>();
+  smem_fft<kLineFFT, kPairThreads, false>(sm, a.tw_l, tid);
   const int lo = a.fsc_bin - a.bw_bins, hi = a.fsc_bin + a.bw_bins;
   const float scale = 1.0f / (float)kLineFFT;
-  for (int k = lane; k < kLineFFT; k += 32) {
+  for (int k = tid; k < kLineFFT; k += kPairThreads) {
     const int kk = k <= kLineFFT / 2 ? k : kLineFFT - k;
     const float m = (kk >= lo && kk <= hi) ? scale : 0.0f;
     const float2 x = sm[pidx(k)];
     sm[pidx(k)] = make_float2(x.x * m, x.y * m);
   }
-  __syncwarp();
-  smem_fft<kLineFFT, 32, true>(sm, a.tw_l_inv, opaque_index(lane));
+  fft_sync<kPairThreads>();
+  smem_fft<kLineFFT, kPairThreads, true>(sm, a.tw_l_inv, opaque_index(tid));
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
+// Sums of K values over a pair's threads, the same in every thread: each
+// warp's butterfly, then warp 0 + warp 1.  red is the pair's, free again
+// after the caller's next pair barrier.
+template <int K>
+__device__ __forceinline__ void pair_sum(double (&v)[K], double (*red)[8], int tid) {
+  static_assert(K <= 8, "red holds 8 sums a warp");
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
+  if ((tid & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < K; k++) red[tid >> 5][k] = v[k];
+  fft_sync<kPairThreads>();
+#pragma unroll
+  for (int k = 0; k < K; k++) v[k] = red[0][k] + red[1][k];
 }
 
-// One warp per pair of chroma lines.  MODE 0: forward; 1: forward + backward.
+// Two warps per pair of chroma lines.  MODE 0: forward; 1: forward + backward.
 // Each line's gain is the decoder's ACC, recomputed from the band-passed
 // burst at the current parameters (g = ref / rms over the burst window), so
 // the backward pass also carries dL/dg back into the burst samples.
+// Latency bound (FP64 coordinates and sums, two transforms each way, a few MB
+// of traffic): a warp a pair at 146 registers put 1.8 CTAs of four warps on an
+// SM; two warps halve each thread's columns.  The gradient of 8 fields 107 ->
+// 69 us, the planes of 4 fields 64 -> 39 us.
 template <int MODE>
-__global__ void __launch_bounds__(32 * kLineWarps) adj_chroma_kernel(AdjArgs a) {
-  __shared__ float2 sm_all[kLineWarps][fft_pad(kLineFFT)];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float2* sm = sm_all[warp];
+__global__ void __launch_bounds__(kPairThreads * kPairs) adj_chroma_kernel(AdjArgs a) {
+  __shared__ float2 sm_all[kPairs][fft_pad(kLineFFT)];
+  __shared__ double red_all[kPairs][3][2][8];
+  const int g = threadIdx.x / kPairThreads, tid = threadIdx.x % kPairThreads;
+  float2* sm = sm_all[g];
+  double(*red)[2][8] = red_all[g];
   const int nlines = a.fields * a.out_h;
-  const int la = 2 * (blockIdx.x * kLineWarps + warp), lb = la + 1;
-  if (la >= nlines) return;  // whole warp
+  const int la = 2 * (blockIdx.x * kPairs + g), lb = la + 1;
+  if (la >= nlines) return;  // the pair's warps leave together
   const bool has_b = lb < nlines;
   const int W = a.out_w;
-  for (int c = lane; c < kLineFFT; c += 32) {
+#pragma unroll 4
+  for (int c = tid; c < kLineFFT; c += kPairThreads) {
     float xa = 0.0f, xb = 0.0f;
     if (c < W) {
       const ChromaSample sa = chroma_sample(a, la, c);
@@ -234,32 +291,33 @@ __global__ void __launch_bounds__(32 * kLineWarps) adj_chroma_kernel(AdjArgs a) 
     }
     sm[pidx(c)] = make_float2(xa, xb);
   }
-  line_bandpass(sm, a, lane);
+  line_bandpass(sm, a, tid);
   // ACC gains from the burst window
-  double ssa = 0.0, ssb = 0.0;
-  for (int i = lane; i < kBurstLen; i += 32) {
+  double ss[2] = {0.0, 0.0};
+  for (int i = tid; i < kBurstLen; i += kPairThreads) {
     const float2 v = sm[pidx(a.burst_start + i)];
-    ssa += (double)v.x * v.x;
-    ssb += (double)v.y * v.y;
+    ss[0] += (double)v.x * v.x;
+    ss[1] += (double)v.y * v.y;
   }
-  ssa = warp_sum(ssa);
-  ssb = warp_sum(ssb);
-  const double rms_a = sqrt(ssa / kBurstLen), rms_b = sqrt(ssb / kBurstLen);
+  pair_sum(ss, red[0], tid);
+  const double rms_a = sqrt(ss[0] / kBurstLen), rms_b = sqrt(ss[1] / kBurstLen);
   const double ga = rms_a > 1.0 ? (double)a.burst_abs_ref / rms_a : 0.0;
   const double gb = (has_b && rms_b > 1.0) ? (double)a.burst_abs_ref / rms_b : 0.0;
-  if (lane == 0) {
+  if (tid == 0) {
     a.gain_out[la] = (float)ga;
     if (has_b) a.gain_out[lb] = (float)gb;
   }
   const int ra = la % a.out_h, rb = lb % a.out_h;
   const bool loss_a = ra >= a.row0 && ra < a.row1 && ra + 1 < a.lpf;
   const bool loss_b = has_b && rb >= a.row0 && rb < a.row1 && rb + 1 < a.lpf;
-  double la_loss = 0.0, lb_loss = 0.0, dga = 0.0, dgb = 0.0;
-  // dL/dC per column, kept per lane
-  constexpr int kPerLane = (kLineFFT + 31) / 32;  // columns per lane (out_w <= kLineFFT)
-  float ea[kPerLane], eb[kPerLane];
-  int n = 0;
-  for (int c = lane; c < W; c += 32, n++) {
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};  // losses, dL/dgains
+  // dL/dC per column, kept per thread
+  float ea[kPerThread], eb[kPerThread];
+#pragma unroll
+  for (int n = 0; n < kPerThread; n++) {
+    const int c = tid + kPairThreads * n;
+    ea[n] = eb[n] = 0.0f;
+    if (c >= W) continue;
     const float2 v = sm[pidx(c)];
     const size_t pa = (size_t)la * W + c, pb = (size_t)lb * W + c;
     const double Ca = ga * (double)v.x + 32768.0, Cb = gb * (double)v.y + 32768.0;
@@ -270,38 +328,34 @@ __global__ void __launch_bounds__(32 * kLineWarps) adj_chroma_kernel(AdjArgs a) 
     const bool col = c >= a.col0 && c < a.col1;
     const double da = loss_a && col ? Ca - (double)__ldg(&a.tgt_c[pa]) : 0.0;
     const double db = loss_b && col ? Cb - (double)__ldg(&a.tgt_c[pb]) : 0.0;
-    la_loss += da * da;
-    lb_loss += db * db;
+    acc[0] += da * da;
+    acc[1] += db * db;
     const double gca = 2.0 * da * a.inv_nc, gcb = 2.0 * db * a.inv_nc;
     ea[n] = (float)gca;
     eb[n] = (float)gcb;
-    dga += gca * (double)v.x;  // dL/dgain
-    dgb += gcb * (double)v.y;
+    acc[2] += gca * (double)v.x;  // dL/dgain
+    acc[3] += gcb * (double)v.y;
   }
-  la_loss = warp_sum(la_loss);
-  lb_loss = warp_sum(lb_loss);
+  pair_sum(acc, red[1], tid);  // its barrier ends every read of the band-passed lines but a thread's own
   double* rpa = a.row + (size_t)la * kAdjRowVals;
   double* rpb = a.row + (size_t)lb * kAdjRowVals;
-  if (lane == 0) {
-    rpa[kRowLossC] = la_loss;
-    if (has_b) rpb[kRowLossC] = lb_loss;
+  if (tid == 0) {
+    rpa[kRowLossC] = acc[0];
+    if (has_b) rpb[kRowLossC] = acc[1];
   }
   if (MODE == 0) return;
-  dga = warp_sum(dga);
-  dgb = warp_sum(dgb);
   // dL/d(band-passed line) = g dL/dC + dL/dg dg/dbp, with dg/dbp_i = -g bp_i / ss
   // on the burst window
-  const double ka = ssa > 0.0 && ga > 0.0 ? -dga * ga / ssa : 0.0;
-  const double kb = ssb > 0.0 && gb > 0.0 ? -dgb * gb / ssb : 0.0;
-  __syncwarp();
-  n = 0;
-  for (int c = lane; c < kLineFFT; c += 32) {
+  const double ka = ss[0] > 0.0 && ga > 0.0 ? -acc[2] * ga / ss[0] : 0.0;
+  const double kb = ss[1] > 0.0 && gb > 0.0 ? -acc[3] * gb / ss[1] : 0.0;
+#pragma unroll
+  for (int n = 0; n < kPerThread; n++) {
+    const int c = tid + kPairThreads * n;
     const float2 bp = sm[pidx(c)];
     double ha = 0.0, hb = 0.0;
     if (c < W) {
       ha = ga * (double)ea[n];
       hb = gb * (double)eb[n];
-      n++;
     }
     if (c >= a.burst_start && c < a.burst_start + kBurstLen) {
       ha += ka * (double)bp.x;
@@ -309,41 +363,37 @@ __global__ void __launch_bounds__(32 * kLineWarps) adj_chroma_kernel(AdjArgs a) 
     }
     sm[pidx(c)] = make_float2((float)ha, (float)hb);
   }
-  line_bandpass(sm, a, lane);  // BP is symmetric: its own adjoint
-  double ph_a = 0.0, ph_b = 0.0, x0a = 0.0, x1a = 0.0, x0b = 0.0, x1b = 0.0;
-  for (int c = lane; c < W; c += 32) {
+  line_bandpass(sm, a, tid);  // BP is symmetric: its own adjoint
+  double grad[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // phase, x0, x1 of line a, then b
+#pragma unroll 4
+  for (int c = tid; c < W; c += kPairThreads) {
     const float2 h = sm[pidx(c)];
     const ChromaSample sa = chroma_sample(a, la, c);
     if (sa.s.ok) {
-      ph_a += (double)h.x * (double)sa.s.v * (double)sa.sn;
+      grad[0] += (double)h.x * (double)sa.s.v * (double)sa.sn;
       const double gx = (double)h.x * (double)sa.het * (double)sa.s.dv;
-      x0a += gx * (1.0 - sa.fc);
-      x1a += gx * sa.fc;
+      grad[1] += gx * (1.0 - sa.fc);
+      grad[2] += gx * sa.fc;
     }
     if (has_b) {
       const ChromaSample sb = chroma_sample(a, lb, c);
       if (sb.s.ok) {
-        ph_b += (double)h.y * (double)sb.s.v * (double)sb.sn;
+        grad[3] += (double)h.y * (double)sb.s.v * (double)sb.sn;
         const double gx = (double)h.y * (double)sb.het * (double)sb.s.dv;
-        x0b += gx * (1.0 - sb.fc);
-        x1b += gx * sb.fc;
+        grad[4] += gx * (1.0 - sb.fc);
+        grad[5] += gx * sb.fc;
       }
     }
   }
-  ph_a = warp_sum(ph_a);
-  x0a = warp_sum(x0a);
-  x1a = warp_sum(x1a);
-  ph_b = warp_sum(ph_b);
-  x0b = warp_sum(x0b);
-  x1b = warp_sum(x1b);
-  if (lane == 0) {
-    rpa[kRowPhase] = ph_a;
-    rpa[kRowChromaX0] = x0a;
-    rpa[kRowChromaX1] = x1a;
+  pair_sum(grad, red[2], tid);
+  if (tid == 0) {
+    rpa[kRowPhase] = grad[0];
+    rpa[kRowChromaX0] = grad[1];
+    rpa[kRowChromaX1] = grad[2];
     if (has_b) {
-      rpb[kRowPhase] = ph_b;
-      rpb[kRowChromaX0] = x0b;
-      rpb[kRowChromaX1] = x1b;
+      rpb[kRowPhase] = grad[3];
+      rpb[kRowChromaX0] = grad[4];
+      rpb[kRowChromaX1] = grad[5];
     }
   }
 }
@@ -353,12 +403,17 @@ __global__ void __launch_bounds__(32 * kLineWarps) adj_chroma_kernel(AdjArgs a) 
 // the block's outputs, zero elsewhere); dL/dtheta_j = sum_k Re(X[k] dG_j[k]
 // conj(W[k])).  The two transforms are separate: the demod (~1e5 Hz with a
 // large DC term) and the gradient differ by many orders of magnitude, so
-// packing them into one FP32 transform would bury W in X's rounding.
-__global__ void __launch_bounds__(kT, 1) adj_deemph_kernel(AdjArgs a) {
+// packing them into one FP32 transform would bury W in X's rounding.  X waits
+// in tensor memory while W is transformed, each thread's 32 words in columns
+// of its own, so that two CTAs fit an SM (K1b's arrangement).  8 fields: 56 us;
+// with X in a second 70 KB buffer and one CTA an SM 68 us.
+constexpr int kTmemCols = 32 * (kT / 128);
+__global__ void __launch_bounds__(kT, 2) adj_deemph_kernel(AdjArgs a) {
   extern __shared__ float2 sm[];
-  float2* sx = sm + fft_pad(kN);  // X in natural order
   __shared__ double sh[kT / 32 * 4];
-  const int t = threadIdx.x;
+  __shared__ uint32_t tmem_base;
+  const int t = threadIdx.x, warp = t >> 5;
+  tmem_alloc<kTmemCols>(&tmem_base, warp);
   const long long j0 = (long long)blockIdx.x * a.b_out;
   float2 v[16];
 #pragma unroll
@@ -367,34 +422,50 @@ __global__ void __launch_bounds__(kT, 1) adj_deemph_kernel(AdjArgs a) {
     v[q] = make_float2(p >= 0 && p < a.total ? __ldg(&a.dem[p]) : 0.0f, 0.0f);
   }
   RegFFT<kN>::run<false>(v, sm, a.tw_b, t);
+  const uint32_t own = tmem_own(tmem_base, warp, 32);
 #pragma unroll
-  for (int q = 0; q < 16; q++) sx[pidx(t + kT * q)] = v[q];
+  for (int c = 0; c < 4; c++) {
+    const float2 x[4] = {v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]};
+    tmem_st8(own + 8 * c, x);
+  }
+  tmem_wait_st();
 #pragma unroll
   for (int q = 0; q < 16; q++) {
     const int i = t + kT * q - a.b_pos;
     v[q] = make_float2((i >= 0 && i < a.b_out && j0 + i < a.total) ? __ldg(&a.gvideo[j0 + i]) : 0.0f, 0.0f);
   }
-  RegFFT<kN>::run<false>(v, sm, a.tw_b, t);  // each thread reads back only its own X slots
+  RegFFT<kN>::run<false>(v, sm, a.tw_b, opaque_index(t));
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-  for (int q = 0; q < 16; q++) {
-    const int k = t + kT * q;
-    const float2 x = sx[pidx(k)], w = v[q];
-    const double pr = (double)x.x * w.x + (double)x.y * w.y;  // X conj(W)
-    const double pi = (double)x.y * w.x - (double)x.x * w.y;
+  for (int c = 0; c < 4; c++) {
+    float2 xs[4];
+    tmem_ld8(own + 8 * c, xs);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const float2 d = __ldg(&a.dg[(size_t)j * kN + k]);
-      acc[j] += pr * (double)d.x - pi * (double)d.y;
+    for (int i = 0; i < 4; i++) {
+      const int q = 4 * c + i, k = t + kT * q;
+      const float2 x = xs[i], w = v[q];
+      const double pr = (double)x.x * w.x + (double)x.y * w.y;  // X conj(W)
+      const double pi = (double)x.y * w.x - (double)x.x * w.y;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float2 d = __ldg(&a.dg[(size_t)j * kN + k]);
+        acc[j] += pr * (double)d.x - pi * (double)d.y;
+      }
     }
   }
-  block_sum<kT, 4>(acc, sh);
+  block_sum<kT, 4>(acc, sh);  // its barrier follows every thread's last read of tensor memory
   if (t == 0)
 #pragma unroll
     for (int j = 0; j < 4; j++) a.blk[(size_t)blockIdx.x * 4 + j] = acc[j];
+  tmem_free<kTmemCols>(tmem_base, warp);
 }
 
 }  // namespace
+
+void launch_adj_filter(const AdjFilterArgs& a, cudaStream_t st) {
+  static_assert(kN % kFilterThreads == 0, "a thread per bin");
+  adj_filter_kernel<<<kN / kFilterThreads, kFilterThreads, 0, st>>>(a);
+}
 
 void launch_adj_video(const AdjArgs& a, cudaStream_t st) {
   const size_t smem = sizeof(float2) * fft_pad(kN);
@@ -410,13 +481,13 @@ void launch_adj_luma(const AdjArgs& a, int mode, cudaStream_t st) {
 
 void launch_adj_chroma(const AdjArgs& a, int mode, cudaStream_t st) {
   const int pairs = (a.fields * a.out_h + 1) / 2;
-  const int grid = (pairs + kLineWarps - 1) / kLineWarps;
-  if (mode == 1) adj_chroma_kernel<1><<<grid, 32 * kLineWarps, 0, st>>>(a);
-  else adj_chroma_kernel<0><<<grid, 32 * kLineWarps, 0, st>>>(a);
+  const int grid = (pairs + kPairs - 1) / kPairs;
+  if (mode == 1) adj_chroma_kernel<1><<<grid, kPairThreads * kPairs, 0, st>>>(a);
+  else adj_chroma_kernel<0><<<grid, kPairThreads * kPairs, 0, st>>>(a);
 }
 
 void launch_adj_deemph(const AdjArgs& a, cudaStream_t st) {
-  const size_t smem = 2 * sizeof(float2) * fft_pad(kN);
+  const size_t smem = sizeof(float2) * fft_pad(kN);
   cudaFuncSetAttribute(adj_deemph_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   adj_deemph_kernel<<<a.blocks, kT, smem, st>>>(a);
 }

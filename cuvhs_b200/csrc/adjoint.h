@@ -71,6 +71,18 @@ struct AdjArgs {
   double* blk;               // [blocks * 4]
 };
 
+// Block spectrum of the video filter H(z) S(f), H = (n0 + n1 z^-1 + n2 z^-2) /
+// (1 + m1 z^-1 + m2 z^-2) with n0 = 1 + m1 + m2 - n1 - n2, on the kNb grid, / kNb,
+// and (dg not null) its derivatives by n1, n2, m1, m2; all in FP64, rounded
+// once.  z1[k] = e^{-2 pi i k / kNb}, s[k] = S at bin k's frequency.
+struct AdjFilterArgs {
+  double n1, n2, m1, m2;
+  const double2* z1;
+  const double* s;
+  float2* gv;
+  float2* dg;
+};
+void launch_adj_filter(const AdjFilterArgs& a, cudaStream_t st);
 void launch_adj_video(const AdjArgs& a, cudaStream_t st);
 // mode 0: forward (loss, optional planes); 1: forward + backward
 void launch_adj_luma(const AdjArgs& a, int mode, cudaStream_t st);

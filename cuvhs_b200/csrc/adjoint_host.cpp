@@ -2,7 +2,7 @@
 // cuvhs_adjoint_*).  The device kernels are in adjoint.cu.
 //
 // The video filter's block spectrum and its four parameter derivatives are
-// built here in FP64 for every call, directly on the 8192-point block grid:
+// built on the device in FP64 for every call, directly on the 8192-point block grid:
 // the response R = H(z) S(f) there is the spectrum of the filter's time
 // kernel wrapped to 8192 samples, whose taps beyond the +/-b_pos support of
 // the overlap-save blocks (the support the decoder's K1b uses) are below
@@ -61,12 +61,16 @@ struct cuvhs_adjoint {
   bool has_target = false;
   double nominal[4] = {0, 0, 0, 0};
   std::string err;
-  // host staging
-  std::vector<double> h_row, h_blk;
-  std::vector<float2> h_gv, h_dg;
+  double2* d_z1 = nullptr;  // [kN] e^{-2 pi i k / kN}
+  double* d_s = nullptr;    // [kN] the super-Gaussian at each bin
+  // page-locked host staging of d_row and d_blk
+  double *h_row = nullptr, *h_blk = nullptr;
+  size_t n_row = 0, n_blk = 0;
 
   ~cuvhs_adjoint() {
     for (void* p : allocs) cudaFree(p);
+    if (h_row) cudaFreeHost(h_row);
+    if (h_blk) cudaFreeHost(h_blk);
     if (ctx) cuvhs_destroy(ctx);
   }
   template <typename T>
@@ -81,40 +85,29 @@ struct cuvhs_adjoint {
   }
   cuvhs::Context& c() { return ctx->c; }
 
-  // Block spectrum of the video filter for (n1, n2, m1, m2) and its derivatives.
-  void build_filter(const double th[4]) {
+  // Block spectrum of the video filter for (n1, n2, m1, m2) and, on request, its derivatives.
+  void build_filter(const double th[4], bool derivs) {
+    cuvhs::launch_adj_filter({th[0], th[1], th[2], th[3], d_z1, d_s, d_gv, derivs ? d_dg : nullptr}, c().stream);
+  }
+
+  // The parameter-free tables of the filter (once per model).
+  void upload_filter_tables() {
     const double fs = c().fmt.fs_hz;
-    const double n1 = th[0], n2 = th[1], m1 = th[2], m2 = th[3];
-    const double n0 = 1.0 + m1 + m2 - n1 - n2;
-    std::vector<cd> R(kN), dR[4];
-    for (auto& v : dR) v.assign(kN, cd(0.0, 0.0));
+    std::vector<double2> z(kN);
+    std::vector<double> s(kN);
     for (int k = 0; k < kN; k++) {
       const int kk = k <= kN / 2 ? k : k - kN;
-      const double w = 2.0 * kPi * (double)kk / (double)kN;
-      const cd z1 = std::exp(cd(0.0, -w)), z2 = z1 * z1;
-      const cd num = n0 + n1 * z1 + n2 * z2, den = 1.0 + m1 * z1 + m2 * z2;
-      const cd H = num / den;
-      const double S = super_gauss(std::fabs((double)kk) * fs / (double)kN, 3.0e6, 9);
-      R[k] = H * S;
-      dR[0][k] = (z1 - 1.0) / den * S;            // n0 moves with n1
-      dR[1][k] = (z2 - 1.0) / den * S;
-      dR[2][k] = (1.0 / den - H * z1 / den) * S;  // n0 moves with m1
-      dR[3][k] = (1.0 / den - H * z2 / den) * S;
+      const cd z1 = std::exp(cd(0.0, -2.0 * kPi * (double)kk / (double)kN));
+      z[k] = make_double2(z1.real(), z1.imag());
+      s[k] = super_gauss(std::fabs((double)kk) * fs / (double)kN, 3.0e6, 9);
     }
-    h_gv.resize(kN);
-    h_dg.resize((size_t)4 * kN);
-    for (int k = 0; k < kN; k++) {
-      h_gv[k] = make_float2((float)(R[k].real() / kN), (float)(R[k].imag() / kN));
-      for (int j = 0; j < 4; j++)
-        h_dg[(size_t)j * kN + k] = make_float2((float)(dR[j][k].real() / kN), (float)(dR[j][k].imag() / kN));
-    }
+    cudaMemcpy(d_z1, z.data(), sizeof(double2) * kN, cudaMemcpyHostToDevice);
+    cudaMemcpy(d_s, s.data(), sizeof(double) * kN, cudaMemcpyHostToDevice);
   }
 
   void upload_params(const cuvhs_adjoint_params* p, bool derivs) {
-    build_filter(p->deemph);
+    build_filter(p->deemph, derivs);
     cudaStream_t st = c().stream;
-    cudaMemcpyAsync(d_gv, h_gv.data(), sizeof(float2) * kN, cudaMemcpyHostToDevice, st);
-    if (derivs) cudaMemcpyAsync(d_dg, h_dg.data(), sizeof(float2) * 4 * kN, cudaMemcpyHostToDevice, st);
     const int H = c().fmt.output_field_lines;
     cudaMemcpyAsync(d_off, p->line_offset, sizeof(double) * P * (H + 1), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(d_phase, p->chroma_phase, sizeof(double) * P * H, cudaMemcpyHostToDevice, st);
@@ -185,8 +178,15 @@ cuvhs_status cuvhs_adjoint_create(const cuvhs_config* cfg, const uint8_t* sample
   a->d_track = a->alloc<int>(P, ok);
   a->d_gv = a->alloc<float2>(kN, ok);
   a->d_dg = a->alloc<float2>((size_t)4 * kN, ok);
+  a->d_z1 = a->alloc<double2>(kN, ok);
+  a->d_s = a->alloc<double>(kN, ok);
+  a->n_row = (size_t)P * H * cuvhs::kAdjRowVals;
+  a->n_blk = (size_t)a->blocks * 4;
+  ok = ok && cudaHostAlloc((void**)&a->h_row, sizeof(double) * a->n_row, cudaHostAllocDefault) == cudaSuccess &&
+       cudaHostAlloc((void**)&a->h_blk, sizeof(double) * a->n_blk, cudaHostAllocDefault) == cudaSuccess;
   if (!ok) {
-    fprintf(stderr, "cuvhs_adjoint_create: device allocation failed\n");
+    cudaGetLastError();
+    fprintf(stderr, "cuvhs_adjoint_create: allocation failed\n");
     delete a;
     return CUVHS_ERR_OUT_OF_MEMORY;
   }
@@ -267,8 +267,8 @@ cuvhs_status cuvhs_adjoint_create(const cuvhs_config* cfg, const uint8_t* sample
     a->nominal[3] = b2 / b0;
   }
   // one pass at the nominal parameters leaves the ACC gains for inspection
-  a->build_filter(a->nominal);
-  cudaMemcpyAsync(a->d_gv, a->h_gv.data(), sizeof(float2) * kN, cudaMemcpyHostToDevice, st);
+  a->upload_filter_tables();
+  a->build_filter(a->nominal, false);
   cudaMemsetAsync(a->d_tgt_c, 0, sizeof(float) * P * H * W, st);
   cuvhs::launch_adj_video(g, st);
   cuvhs::launch_adj_chroma(g, 0, st);
@@ -277,8 +277,6 @@ cuvhs_status cuvhs_adjoint_create(const cuvhs_config* cfg, const uint8_t* sample
     delete a;
     return CUVHS_ERR_CUDA;
   }
-  a->h_row.resize((size_t)P * H * cuvhs::kAdjRowVals);
-  a->h_blk.resize((size_t)a->blocks * 4);
   *out = a;
   return CUVHS_OK;
 }
@@ -335,14 +333,14 @@ cuvhs_status cuvhs_adjoint_fwd(cuvhs_adjoint* a, const cuvhs_adjoint_params* p, 
   g.deviation = p->deviation;
   g.y_out = luma ? a->d_y : nullptr;
   g.c_out = chroma ? a->d_c : nullptr;
-  cudaMemsetAsync(a->d_row, 0, sizeof(double) * a->h_row.size(), st);
+  cudaMemsetAsync(a->d_row, 0, sizeof(double) * a->n_row, st);
   cuvhs::launch_adj_video(g, st);
   cuvhs::launch_adj_luma(g, 0, st);
   cuvhs::launch_adj_chroma(g, 0, st);
   const size_t np = (size_t)a->P * CUVHS_FIELD_HEIGHT * CUVHS_FIELD_WIDTH;
   if (luma) cudaMemcpyAsync(luma, a->d_y, sizeof(float) * np, cudaMemcpyDeviceToHost, st);
   if (chroma) cudaMemcpyAsync(chroma, a->d_c, sizeof(float) * np, cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(a->h_row.data(), a->d_row, sizeof(double) * a->h_row.size(), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(a->h_row, a->d_row, sizeof(double) * a->n_row, cudaMemcpyDeviceToHost, st);
   if (!a->finish("adjoint forward")) return CUVHS_ERR_CUDA;
   if (loss) *loss = sum_loss(a);
   return CUVHS_OK;
@@ -357,18 +355,18 @@ cuvhs_status cuvhs_adjoint_bwd(cuvhs_adjoint* a, const cuvhs_adjoint_params* p, 
   cuvhs::AdjArgs g = a->args;
   g.carrier = p->carrier_hz;
   g.deviation = p->deviation;
-  cudaMemsetAsync(a->d_row, 0, sizeof(double) * a->h_row.size(), st);
+  cudaMemsetAsync(a->d_row, 0, sizeof(double) * a->n_row, st);
   cudaMemsetAsync(a->d_gvideo, 0, sizeof(float) * a->total, st);
   cuvhs::launch_adj_video(g, st);  // recomputed: the forward keeps nothing for the backward
   cuvhs::launch_adj_luma(g, 1, st);
   cuvhs::launch_adj_chroma(g, 1, st);
   cuvhs::launch_adj_deemph(g, st);
-  cudaMemcpyAsync(a->h_row.data(), a->d_row, sizeof(double) * a->h_row.size(), cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(a->h_blk.data(), a->d_blk, sizeof(double) * a->h_blk.size(), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(a->h_row, a->d_row, sizeof(double) * a->n_row, cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(a->h_blk, a->d_blk, sizeof(double) * a->n_blk, cudaMemcpyDeviceToHost, st);
   if (!a->finish("adjoint backward")) return CUVHS_ERR_CUDA;
   if (loss) *loss = sum_loss(a);
   const int H = CUVHS_FIELD_HEIGHT;
-  const double* R = a->h_row.data();
+  const double* R = a->h_row;
   auto row = [&](int f, int r, int k) { return R[((size_t)f * H + r) * cuvhs::kAdjRowVals + k]; };
   double dcar = 0.0, ddev = 0.0;
   for (int f = 0; f < a->P; f++)
