@@ -199,6 +199,7 @@ struct GuardArgs {
   int cap;
   double* values;  // optional [cap]: the FP64 sync value of each listed sample
   int* flips = nullptr;  // optional: counts samples whose FP64 side differs from their FP32 value's
+  unsigned* pulse_bits = nullptr;  // optional: K1b's in-pulse bits, corrected with the samples that flip
   long long* dbg_clk = nullptr;  // optional [kGuardClockSamples][kPhaseSlots]: SM clock at each phase of a sample's CTA
 };
 constexpr int kGuardClockSamples = 1024;
@@ -236,10 +237,11 @@ struct EdgeArgs {
   unsigned *fall, *rise;
   int cap;
 };
-void launch_edges_bits(const unsigned* bits, long long total, unsigned* fall, unsigned* rise, int* counts, int cap,
-                       int2* blk, cudaStream_t st);
+// Returns the kernels launched.
+int launch_edges_bits(const unsigned* bits, long long total, unsigned* fall, unsigned* rise, int* counts, int cap,
+                      int2* blk, cudaStream_t st);
 size_t pulse_bit_words(long long total);
-void launch_edges_bits_many(const ArgsMany<EdgeArgs>& e, int portions, long long max_total, cudaStream_t st);
+int launch_edges_bits_many(const ArgsMany<EdgeArgs>& e, int portions, long long max_total, cudaStream_t st);
 void launch_edges(const float* sync, long long total, float thr_rel, unsigned* fall, unsigned* rise,
                   int* counts, int cap, int2* blk, unsigned* masks, cudaStream_t st);
 
@@ -430,6 +432,7 @@ struct LineLocArgs {
   int* is_first;         // [num_fields] 1 first, 0 second (single pass: -1 undetermined)
   long long raw_offset;  // capture position of the chunk
   int single_pass;
+  int pulses_from_edges = 0;  // 1: the per-field pass forms ps/pl/pn itself (launch_field_pulses not needed)
   int *dbg_vs = nullptr, *dbg_vl = nullptr, *dbg_vt = nullptr, *dbg_vn = nullptr;  // optional: validated pulses
   long long* dbg_clk = nullptr;  // optional [num_fields][kPhaseSlots]: SM clock at each phase of a field's CTAs
 };

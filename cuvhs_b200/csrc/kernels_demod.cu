@@ -569,78 +569,140 @@ __global__ void __launch_bounds__(kEdgeThreads) edge_write_kernel(long long tota
   }
 }
 
-// Threshold edges from in-pulse bits: one thread per 32-position word (a CTA
-// 8192 positions).  falling = in now and not before, rising = out now and in
-// before; position 0 counts as preceded by "out" (a pulse open there falls
-// there), positions at or past total hold no bits.
-constexpr int kBitEdgeSeg = kEdgeThreads * 32;
+// Threshold edges from in-pulse bits: WPT consecutive 32-position words a
+// thread (a CTA 8192 * WPT positions).  falling = in now and not before,
+// rising = out now and in before; position 0 counts as preceded by "out" (a
+// pulse open there falls there), positions at or past total hold no bits.
+//
+// A count pass, then a write pass that places each CTA's edges.  Where the
+// CTAs are few (kDirectBlocks), each sums the counts before its own (32 KB from
+// L2 at most); past that a scan kernel does it once.  Four words a thread
+// (kWideEdges) once that still gives every SM two CTAs: a quarter of the CTAs,
+// each with a quarter of the counts to sum (one word a thread, 2,460 CTAs for
+// 40 fields at 28 MHz: 11 us in the write pass).  Latency bound.
+constexpr int kDirectBlocks = 4096;
+constexpr long long kWideEdges = 296ll * 4 * 8192;
+template <int WPT>
+__host__ __device__ constexpr long long bit_edge_seg() { return (long long)kEdgeThreads * WPT * 32; }
 
-__device__ __forceinline__ void bit_edges(const unsigned* __restrict__ bits, long long total, long long w,
-                                          unsigned& fm, unsigned& rm) {
-  const long long p0 = w * 32;
-  fm = rm = 0;
-  if (p0 >= total) return;
-  const unsigned valid = total - p0 >= 32 ? 0xffffffffu : ((1u << (unsigned)(total - p0)) - 1u);
-  const unsigned in = __ldg(&bits[w]) & valid;
-  const unsigned prev = w > 0 ? (__ldg(&bits[w - 1]) >> 31) : 0u;
-  const unsigned before = (in << 1) | prev;  // bit j: in at position j - 1
-  fm = in & ~before;
-  rm = ~in & before & valid;
+template <int WPT>
+__device__ __forceinline__ void bit_edges(const unsigned* __restrict__ bits, long long total, long long w0,
+                                          unsigned (&fm)[WPT], unsigned (&rm)[WPT]) {
+  unsigned prev = w0 > 0 && w0 * 32 < total ? (__ldg(&bits[w0 - 1]) >> 31) : 0u;
+#pragma unroll
+  for (int q = 0; q < WPT; q++) {
+    const long long w = w0 + q, p0 = w * 32;
+    fm[q] = rm[q] = 0;
+    if (p0 >= total) continue;
+    const unsigned valid = total - p0 >= 32 ? 0xffffffffu : ((1u << (unsigned)(total - p0)) - 1u);
+    const unsigned word = __ldg(&bits[w]), in = word & valid;
+    const unsigned before = (in << 1) | prev;  // bit j: in at position j - 1
+    fm[q] = in & ~before;
+    rm[q] = ~in & before & valid;
+    prev = word >> 31;
+  }
+}
+template <int WPT>
+__device__ __forceinline__ int bit_count(const unsigned (&m)[WPT]) {
+  int n = 0;
+#pragma unroll
+  for (int q = 0; q < WPT; q++) n += __popc(m[q]);
+  return n;
 }
 
-template <class Src>
+template <int WPT, class Src>
 __global__ void __launch_bounds__(kEdgeThreads) edge_bits_count_kernel(const __grid_constant__ Src src) {
   const EdgeArgs& e = src.get();
-  if ((long long)blockIdx.x * kBitEdgeSeg >= e.total) return;  // whole CTA
+  if ((long long)blockIdx.x * bit_edge_seg<WPT>() >= e.total) return;  // whole CTA
   chain_wait();
-  const long long w = (long long)blockIdx.x * kEdgeThreads + threadIdx.x;
-  unsigned fm, rm;
-  bit_edges(e.bits, e.total, w, fm, rm);
+  const long long w = ((long long)blockIdx.x * kEdgeThreads + threadIdx.x) * WPT;
+  unsigned fm[WPT], rm[WPT];
+  bit_edges<WPT>(e.bits, e.total, w, fm, rm);
   int pa, pb;
-  const int2 tot = block_scan2(__popc(fm), __popc(rm), pa, pb);
+  const int2 tot = block_scan2(bit_count(fm), bit_count(rm), pa, pb);
   if (threadIdx.x == 0) e.blk[blockIdx.x] = tot;
 }
 
-template <class Src>
+template <int WPT, class Src>
 __global__ void __launch_bounds__(kScanThreads) edge_bits_scan_kernel(const __grid_constant__ Src src) {
   const EdgeArgs& e = src.get();
-  scan_blocks(e.blk, (int)((e.total + kBitEdgeSeg - 1) / kBitEdgeSeg), e.counts);
+  scan_blocks(e.blk, (int)((e.total + bit_edge_seg<WPT>() - 1) / bit_edge_seg<WPT>()), e.counts);
 }
 
-template <class Src>
+// DIRECT: blk holds the count pass's counts and this CTA sums those before
+// its own (the last CTA writes the totals); else blk holds offsets.
+template <int WPT, bool DIRECT, class Src>
 __global__ void __launch_bounds__(kEdgeThreads) edge_bits_write_kernel(const __grid_constant__ Src src) {
   const EdgeArgs& e = src.get();
-  if ((long long)blockIdx.x * kBitEdgeSeg >= e.total) return;  // whole CTA
+  if ((long long)blockIdx.x * bit_edge_seg<WPT>() >= e.total) return;  // whole CTA
   chain_wait();
-  const long long w = (long long)blockIdx.x * kEdgeThreads + threadIdx.x;
-  unsigned fm, rm;
-  bit_edges(e.bits, e.total, w, fm, rm);
+  const long long w = ((long long)blockIdx.x * kEdgeThreads + threadIdx.x) * WPT;
+  unsigned fm[WPT], rm[WPT];
+  bit_edges<WPT>(e.bits, e.total, w, fm, rm);
   int pa, pb;
-  block_scan2(__popc(fm), __popc(rm), pa, pb);
-  int kf = e.blk[blockIdx.x].x + pa, kr = e.blk[blockIdx.x].y + pb;
-  const long long p0 = w * 32;
-  while (fm) {
-    const int j = __ffs(fm) - 1;
-    fm &= fm - 1;
-    if (kf < e.cap) e.fall[kf] = (unsigned)(p0 + j);
-    kf++;
+  const int2 own = block_scan2(bit_count(fm), bit_count(rm), pa, pb);
+  int2 at;
+  if constexpr (DIRECT) {
+    int sa = 0, sb = 0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += kEdgeThreads) {
+      const int2 c = __ldcg(&e.blk[b]);
+      sa += c.x;
+      sb += c.y;
+    }
+    int ia, ib;
+    __syncthreads();  // the first scan's totals
+    at = block_scan2(sa, sb, ia, ib);
+    if (threadIdx.x == 0 && (long long)(blockIdx.x + 1) * bit_edge_seg<WPT>() >= e.total) {
+      e.counts[0] = at.x + own.x;
+      e.counts[1] = at.y + own.y;
+    }
+  } else {
+    at = e.blk[blockIdx.x];
   }
-  while (rm) {
-    const int j = __ffs(rm) - 1;
-    rm &= rm - 1;
-    if (kr < e.cap) e.rise[kr] = (unsigned)(p0 + j);
-    kr++;
+  int kf = at.x + pa, kr = at.y + pb;
+#pragma unroll
+  for (int q = 0; q < WPT; q++) {
+    const long long p0 = (w + q) * 32;
+    for (unsigned m = fm[q]; m; m &= m - 1) {
+      if (kf < e.cap) e.fall[kf] = (unsigned)(p0 + __ffs(m) - 1);
+      kf++;
+    }
+    for (unsigned m = rm[q]; m; m &= m - 1) {
+      if (kr < e.cap) e.rise[kr] = (unsigned)(p0 + __ffs(m) - 1);
+      kr++;
+    }
   }
+}
+
+// The passes over `portions` captures of at most max_total positions.
+template <int WPT, class S>
+void edges_bits_launch(const S& e, int portions, long long max_total, cudaStream_t st) {
+  const int nblk = (int)((max_total + bit_edge_seg<WPT>() - 1) / bit_edge_seg<WPT>());
+  const dim3 grid(nblk, 1, portions);
+  launch_chained(edge_bits_count_kernel<WPT, S>, grid, dim3(kEdgeThreads), 0, st, e);
+  if (nblk <= kDirectBlocks) {
+    launch_chained(edge_bits_write_kernel<WPT, true, S>, grid, dim3(kEdgeThreads), 0, st, e);
+  } else {
+    launch_chained(edge_bits_scan_kernel<WPT, S>, dim3(1, 1, portions), dim3(kScanThreads), 0, st, e);
+    launch_chained(edge_bits_write_kernel<WPT, false, S>, grid, dim3(kEdgeThreads), 0, st, e);
+  }
+}
+template <class S>
+int edges_bits_any(const S& e, int portions, long long max_total, cudaStream_t st) {
+  static_assert(kWideEdges <= kDirectBlocks * bit_edge_seg<1>(), "narrow passes sum directly");
+  if (max_total <= 0 || portions <= 0) return 0;
+  if (max_total < kWideEdges) edges_bits_launch<1>(e, portions, max_total, st);
+  else edges_bits_launch<4>(e, portions, max_total, st);
+  return max_total <= kDirectBlocks * bit_edge_seg<4>() ? 2 : 3;
 }
 
 }  // namespace
 
 size_t pulse_bit_words(long long total) { return (size_t)((total + 31) / 32) + 1; }
 
-void launch_edges_bits(const unsigned* bits, long long total, unsigned* fall, unsigned* rise, int* counts, int cap,
-                       int2* blk, cudaStream_t st) {
-  const int nblk = (int)((total + kBitEdgeSeg - 1) / kBitEdgeSeg);
-  if (nblk <= 0) return;
+int launch_edges_bits(const unsigned* bits, long long total, unsigned* fall, unsigned* rise, int* counts, int cap,
+                      int2* blk, cudaStream_t st) {
   ArgsOne<EdgeArgs> e;
   e.a[0].bits = bits;
   e.a[0].total = total;
@@ -649,19 +711,11 @@ void launch_edges_bits(const unsigned* bits, long long total, unsigned* fall, un
   e.a[0].fall = fall;
   e.a[0].rise = rise;
   e.a[0].cap = cap;
-  using S = ArgsOne<EdgeArgs>;
-  launch_chained(edge_bits_count_kernel<S>, dim3(nblk), dim3(kEdgeThreads), 0, st, e);
-  launch_chained(edge_bits_scan_kernel<S>, dim3(1), dim3(kScanThreads), 0, st, e);
-  launch_chained(edge_bits_write_kernel<S>, dim3(nblk), dim3(kEdgeThreads), 0, st, e);
+  return edges_bits_any(e, 1, total, st);
 }
 
-void launch_edges_bits_many(const ArgsMany<EdgeArgs>& e, int portions, long long max_total, cudaStream_t st) {
-  const int nblk = (int)((max_total + kBitEdgeSeg - 1) / kBitEdgeSeg);
-  if (nblk <= 0 || portions <= 0) return;
-  using S = ArgsMany<EdgeArgs>;
-  launch_chained(edge_bits_count_kernel<S>, dim3(nblk, 1, portions), dim3(kEdgeThreads), 0, st, e);
-  launch_chained(edge_bits_scan_kernel<S>, dim3(1, 1, portions), dim3(kScanThreads), 0, st, e);
-  launch_chained(edge_bits_write_kernel<S>, dim3(nblk, 1, portions), dim3(kEdgeThreads), 0, st, e);
+int launch_edges_bits_many(const ArgsMany<EdgeArgs>& e, int portions, long long max_total, cudaStream_t st) {
+  return edges_bits_any(e, portions, max_total, st);
 }
 
 void launch_k1a(const DemodArgs& a, int f0, int nf, cudaStream_t st) {

@@ -265,7 +265,10 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
       double x64 = 0.0;
       for (int w = 0; w < kGT / 32; w++) x64 += red[w];
       const bool in_pulse = x64 <= g.thr_hz;  // the reference's FP64 decision
-      if (g.flips && in_pulse != (g.sync[s] <= g.thr_rel)) atomicAdd(g.flips, 1);
+      if (in_pulse != (g.sync[s] <= g.thr_rel)) {
+        if (g.flips) atomicAdd(g.flips, 1);
+        if (g.pulse_bits) atomicXor(&g.pulse_bits[s >> 5], 1u << (s & 31));
+      }
       float r = (float)(x64 - g.ire0);
       if (in_pulse && !(r <= g.thr_rel)) r = g.thr_rel;
       if (!in_pulse && r <= g.thr_rel) r = nextafterf(g.thr_rel, 3.0e38f);

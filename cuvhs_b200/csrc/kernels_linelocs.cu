@@ -74,8 +74,9 @@ __device__ __forceinline__ long long run_end(const LineLocArgs& a, int nrise, in
 // One CTA: VSYNC candidates (runs of 20-35 us, vsync_discover.cu:58-72) in
 // sample order, clustered into field windows (pipeline.cu:1567-1651).
 //
-// Candidates: the falling edges are taken 1024 at a time, one per thread
-// (coalesced), and a block scan appends the candidates in order.  Clustering:
+// Candidates: the falling edges are taken 8192 at a time, eight per thread
+// (coalesced), and a block scan appends the candidates in order (1024 at a
+// time, three barriers each, took 24 us for the 12,000 edges of 40 fields).  Clustering:
 // the reference opens a window at the first candidate and at every later
 // candidate more than half a field past the open window's start (the
 // candidate less five lines), so the window that follows candidate j opens at
@@ -83,6 +84,7 @@ __device__ __forceinline__ long long run_end(const LineLocArgs& a, int nrise, in
 // once by binary search -- and one thread follows that chain from the first
 // candidate, one step per field.
 constexpr int kWinThreads = 1024;
+constexpr int kWinTiles = 8;
 constexpr int kWinSmemCand = 12288;  // candidates clustered in shared memory; more: the serial path
 size_t fieldwin_smem_bytes() { return (size_t)kWinSmemCand * 2 * sizeof(int); }
 
@@ -93,50 +95,59 @@ __global__ void __launch_bounds__(kWinThreads) fieldwin_kernel(const __grid_cons
   extern __shared__ int wsm[];
   int* scand = wsm;                  // [kWinSmemCand] candidate positions
   int* snext = wsm + kWinSmemCand;   // [kWinSmemCand] index of the next window's first candidate
-  __shared__ int warp_tot[kWinThreads / 32];
-  __shared__ int base_s;
+  __shared__ int place[kWinTiles * (kWinThreads / 32)];  // a tile's and warp's candidates: count, then position
+  __shared__ int step_total;
   const int nfall = min(a.counts[0], a.edge_cap), nrise = min(a.counts[1], a.edge_cap);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if (t == 0) {
-    a.win->err = (a.counts[0] > a.edge_cap || a.counts[1] > a.edge_cap) ? 1 : 0;
-    base_s = 0;
-  }
-  __syncthreads();
-  // candidates in order, one tile of falling edges per step (the next tile's
-  // edges are loaded before the current tile's scan)
-  int nf = 0, nr = 0;
-  if (t < nfall) {
-    nf = (int)a.fall[t];
-    nr = t < nrise ? (int)a.rise[t] : 0;
-  }
-  for (int i0 = 0; i0 < nfall; i0 += kWinThreads) {
-    const int i = i0 + t;
-    const long long fpos = (unsigned)nf;
-    const long long end = i < nrise ? (long long)(unsigned)nr : a.total;  // run_end
-    const bool cand = i < nfall && end - fpos >= a.minw && end - fpos <= a.maxw;
-    const int j = i + kWinThreads;
-    if (j < nfall) {
-      nf = (int)a.fall[j];
-      nr = j < nrise ? (int)a.rise[j] : 0;
+  if (t == 0) a.win->err = (a.counts[0] > a.edge_cap || a.counts[1] > a.edge_cap) ? 1 : 0;
+  // candidates in order: kWinTiles tiles of 1024 falling edges a step, every
+  // load of a step in flight, each tile's and warp's count placed by one scan
+  int base = 0;
+  for (int i0 = 0; i0 < nfall; i0 += kWinTiles * kWinThreads) {
+    unsigned fpos[kWinTiles], rpos[kWinTiles];
+#pragma unroll
+    for (int j = 0; j < kWinTiles; j++) {
+      const int i = i0 + j * kWinThreads + t;
+      fpos[j] = i < nfall ? a.fall[i] : 0u;
+      rpos[j] = i < nfall && i < nrise ? a.rise[i] : 0u;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, cand);
-    if (lane == 0) warp_tot[warp] = __popc(m);
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int w = 0; w < kWinThreads / 32; w++) {
-      if (w < warp) before += warp_tot[w];
-      total += warp_tot[w];
-    }
-    const int k = base_s + before + __popc(m & ((1u << lane) - 1u));
-    if (cand) {
-      if (k < a.cand_cap) a.cand[k] = (int)fpos;
-      if (k < kWinSmemCand) scand[k] = (int)fpos;
+    unsigned m[kWinTiles];
+#pragma unroll
+    for (int j = 0; j < kWinTiles; j++) {
+      const int i = i0 + j * kWinThreads + t;
+      const long long len = (i < nrise ? (long long)rpos[j] : a.total) - (long long)fpos[j];  // to run_end
+      m[j] = __ballot_sync(0xffffffffu, i < nfall && len >= a.minw && len <= a.maxw);
+      if (lane == 0) place[j * (kWinThreads / 32) + warp] = __popc(m[j]);
     }
     __syncthreads();
-    if (t == 0) base_s += total;
+    if (warp == 0) {
+      constexpr int kPer = kWinTiles * (kWinThreads / 32) / 32;
+      int own[kPer], sum = 0;
+#pragma unroll
+      for (int q = 0; q < kPer; q++) {
+        own[q] = sum;
+        sum += place[lane * kPer + q];
+      }
+      int incl = sum;
+      for (int off = 1; off < 32; off <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += o;
+      }
+#pragma unroll
+      for (int q = 0; q < kPer; q++) place[lane * kPer + q] = incl - sum + own[q];
+      if (lane == 31) step_total = incl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kWinTiles; j++)
+      if ((m[j] >> lane) & 1u) {
+        const int k = base + place[j * (kWinThreads / 32) + warp] + __popc(m[j] & ((1u << lane) - 1u));
+        if (k < a.cand_cap) a.cand[k] = (int)fpos[j];
+        if (k < kWinSmemCand) scand[k] = (int)fpos[j];
+      }
+    base += step_total;
     __syncthreads();
   }
-  const int base = base_s;
   const int ncand = min(base, a.cand_cap);
   const long long spf = a.fmt.samples_per_field, spl = a.fmt.samples_per_line;
   auto off_of = [&](long long pos) { return pos > 5 * spl ? pos - 5 * spl : 0LL; };
@@ -179,36 +190,73 @@ __global__ void __launch_bounds__(kWinThreads) fieldwin_kernel(const __grid_cons
   a.win->next_rel = predicted > margin ? predicted - margin : predicted;
 }
 
-// Grid (num_fields): the pulses of field f's window (sync_pulses.cu:10-58):
-// threshold runs that start after the window start and end within the
-// spp-sample scan, at most kMaxPulses.
+// upper_idx by a whole warp: each step probes 32 places of the range at once,
+// so a list of 20,000 edges takes three dependent reads instead of fifteen.
+__device__ __forceinline__ int upper_idx_warp(const unsigned* a, int n, unsigned v) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, hi = n;  // the answer lies in [lo, hi]
+  while (hi > lo) {
+    const int step = (hi - lo + 31) / 32;
+    const int at = min(lo + lane * step, hi);  // lane 0 probes lo
+    const unsigned gt = __ballot_sync(0xffffffffu, at >= hi || a[at] > v);
+    const int k = gt ? __ffs(gt) - 1 : 32;  // the first probe past v (ascending)
+    if (k == 0) return lo;
+    const int last = lo + (k - 1) * step;  // the last probe at or below v
+    hi = k < 32 ? min(lo + k * step, hi) : hi;
+    lo = last + 1;
+  }
+  return lo;
+}
+
+// The pulses of field f's window (sync_pulses.cu:10-58), by its CTA: threshold
+// runs that start after the window start and end within the spp-sample scan,
+// at most kMaxPulses.  Into global memory and, where given, ps_s and pl_s.
+// Returns their number in every thread.
+__device__ int window_pulses(const LineLocArgs& a, int f, int* ps_s = nullptr, int* pl_s = nullptr) {
+  __shared__ int ends[2], brk;
+  const int t = threadIdx.x;
+  const int nfall = min(a.counts[0], a.edge_cap), nrise = min(a.counts[1], a.edge_cap);
+  const long long off = a.offs[f], lim = off + a.fmt.spp - 1;
+  if (t < 64) {  // first start > off (warp 0), first start > lim (warp 1)
+    const int i = upper_idx_warp(a.fall, nfall, (unsigned)min(t < 32 ? off : lim, (long long)UINT32_MAX));
+    if ((t & 31) == 0) {
+      ends[t >> 5] = i;
+      if (t == 32) brk = i;
+    }
+  }
+  __syncthreads();
+  const int i0 = ends[0], i1 = ends[1];
+  for (int b = i0; b < i1; b += kLT) {
+    const int i = b + t;
+    const bool past = i < i1 && run_end(a, nrise, i) > lim;
+    if (past) atomicMin(&brk, i);
+    if (__syncthreads_or(past)) break;
+  }
+  const int n = max(min(brk - i0, kMaxPulses), 0);
+  int* ps = a.ps + (size_t)f * kMaxPulses;
+  int* pl = a.pl + (size_t)f * kMaxPulses;
+  for (int k = t; k < n; k += kLT) {
+    const unsigned s = a.fall[i0 + k];
+    const int len = (int)(run_end(a, nrise, i0 + k) - (long long)s);
+    ps[k] = (int)s;
+    pl[k] = len;
+    if (ps_s) {
+      ps_s[k] = (int)s;
+      pl_s[k] = len;
+    }
+  }
+  if (t == 0) a.pn[f] = n;
+  return n;
+}
+
+// Grid (num_fields).
 template <class Src>
 __global__ void __launch_bounds__(kLT) pulses_kernel(const __grid_constant__ Src src) {
   const LineLocArgs& a = src.get();
   chain_wait();
-  __shared__ int brk;
   const int f = blockIdx.x;
   if (f >= a.win->fields) return;
-  const int nfall = min(a.counts[0], a.edge_cap), nrise = min(a.counts[1], a.edge_cap);
-  const long long off = a.offs[f], lim = off + a.fmt.spp - 1;
-  const int i0 = upper_idx(a.fall, nfall, (unsigned)min(off, (long long)UINT32_MAX));  // first start > off
-  const int i1 = upper_idx(a.fall, nfall, (unsigned)min(lim, (long long)UINT32_MAX));  // first start > lim
-  if (threadIdx.x == 0) brk = i1;
-  __syncthreads();
-  for (int b = i0; b < i1 && b < brk; b += kLT) {
-    const int i = b + threadIdx.x;
-    if (i < i1 && run_end(a, nrise, i) > lim) atomicMin(&brk, i);
-    __syncthreads();
-  }
-  const int n = min(brk - i0, kMaxPulses);
-  int* ps = a.ps + (size_t)f * kMaxPulses;
-  int* pl = a.pl + (size_t)f * kMaxPulses;
-  for (int k = threadIdx.x; k < n; k += kLT) {
-    const unsigned s = a.fall[i0 + k];
-    ps[k] = (int)s;
-    pl[k] = (int)(run_end(a, nrise, i0 + k) - (long long)s);
-  }
-  if (threadIdx.x == 0) a.pn[f] = max(n, 0);
+  window_pulses(a, f);
 }
 
 // ------------------------------------------------------------ K2b per field
@@ -361,90 +409,104 @@ __device__ bool attempt(const int* ps, const int* pl, int n, int first, const IW
 }
 
 // The same recogniser run by a whole warp on one attempt: lane k holds pulse
-// first + k, and every lane steps the state machine over the lanes' pulses
-// (broadcast by shuffles), so no lane diverges and no step waits on shared
-// memory.  Returns the closing flag, the count and last type, and the kept
-// steps (bit k) with their types (2 bits at 2k).
+// first + k, and the width classes become bit masks over the (at most 26)
+// pulses.  In each state the pulses of its own class are kept as they come and
+// those of no class are passed over, so the warp goes from one pulse that may
+// change the state to the next (find-first-set on the masks) instead of
+// pulse by pulse: about six steps instead of 26, 0.5 us an attempt instead of
+// 3.3.  Returns the closing flag, the count and last type, and the kept
+// steps (bit k) with the two bits of their types.
 struct WarpAttempt {
   bool ok;
   int cnt, last;
-  unsigned keep;
-  unsigned long long types;
+  unsigned keep, type0, type1;
 };
 __device__ WarpAttempt attempt_warp(const int* ps, const int* pl, int n, int first, const IWindows& w, int eq_pulses,
                                     int line_len) {
   const int lane = threadIdx.x & 31;
-  const int end = min(n, first + 26);
-  const int mine = first + lane;
-  const int my_len = mine < end ? pl[mine] : 0, my_start = mine < end ? ps[mine] : 0;
+  const int steps = min(n, first + 26) - first;
+  const bool in = lane < steps;
+  const int my_len = in ? pl[first + lane] : 0, my_start = in ? ps[first + lane] : 0;
+  const unsigned H = __ballot_sync(0xffffffffu, in && in_class(my_len, w.h_lo, w.h_hi));
+  const unsigned E = __ballot_sync(0xffffffffu, in && in_class(my_len, w.e_lo, w.e_hi));
+  const unsigned V = __ballot_sync(0xffffffffu, in && in_class(my_len, w.v_lo, w.v_hi));
   bool done = false, vsync_seen = false;
   const double half = eq_pulses / 2.0;
   long long hold_floor = 0, hold_ceil = 0;
   double pending = -1.0;
-  int cur = kHsync, cnt = 0;
-  unsigned keep_mask = 0;
-  unsigned long long types = 0;
-  const int steps = end - first;
-  for (int k = 0; k < steps; k++) {
-    const int len = __shfl_sync(0xffffffffu, my_len, k);
-    const int start = __shfl_sync(0xffffffffu, my_start, k);
-    int type = -1;
-    const bool h = in_class(len, w.h_lo, w.h_hi), e = in_class(len, w.e_lo, w.e_hi),
-               v = in_class(len, w.v_lo, w.v_hi);
-    switch (cur) {
-      case kHsync:
-        if (h) type = kHsync;
-        else if (e) {
-          type = kEq1;
-          pending = half;
-        } else if (v) {
-          vsync_seen = true;
-          type = kVsync;
-        }
-        break;
-      case kEq1:
-        if (e) type = kEq1;
-        else if (v) {
-          vsync_seen = true;
-          type = kVsync;
-          pending = half;
-        } else if (h) type = kHsync;
-        break;
-      case kVsync:
-        if (e) {
-          type = kEq2;
-          pending = half;
-        } else if (v) type = kVsync;
-        else if ((long long)start > hold_floor && h) type = kHsync;
-        break;
-      case kEq2:
-        if (e) type = kEq2;
-        else if (h) {
-          type = kHsync;
-          done = true;
-        }
-        break;
+  int cur = kHsync;
+  WarpAttempt r{false, 0, 0, 0u, 0u, 0u};
+  auto keep = [&](unsigned bits, int type) {
+    r.keep |= bits;
+    if (type & 1) r.type0 |= bits;
+    if (type & 2) r.type1 |= bits;
+  };
+  unsigned rest = steps > 0 ? 0xffffffffu >> (32 - steps) : 0u;  // pulses not yet passed
+  while (rest) {
+    unsigned stay, event;  // pulses that continue the state; that may change it
+    if (cur == kHsync) {
+      stay = H;
+      event = (E | V) & ~H;
+    } else if (cur == kEq1) {
+      stay = E;
+      event = (V | H) & ~E;
+    } else if (cur == kVsync) {
+      stay = V & ~E;
+      event = E | (H & ~V);
+    } else {
+      stay = E;
+      event = H & ~E;
     }
-    bool kept = type >= 0;
-    if (kept && type != cur) {
-      if ((long long)start < hold_ceil) {
-        kept = false;
-      } else if (pending > 0.0) {
+    event &= rest;
+    const unsigned bit = event & (0u - event);  // the first event
+    keep(stay & rest & (bit ? bit - 1u : 0xffffffffu), cur);
+    if (!bit) break;
+    rest &= ~(bit | (bit - 1u));
+    const int start = __shfl_sync(0xffffffffu, my_start, __ffs(bit) - 1);
+    int type;
+    if (cur == kHsync) {
+      if (E & bit) {
+        type = kEq1;
+        pending = half;
+      } else {
+        vsync_seen = true;
+        type = kVsync;
+      }
+    } else if (cur == kEq1) {
+      if (V & bit) {
+        vsync_seen = true;
+        type = kVsync;
+        pending = half;
+      } else {
+        type = kHsync;
+      }
+    } else if (cur == kVsync) {
+      if (E & bit) {
+        type = kEq2;
+        pending = half;
+      } else {
+        type = (long long)start > hold_floor ? kHsync : -1;
+      }
+    } else {
+      type = kHsync;
+      done = true;
+    }
+    if (type >= 0 && (long long)start >= hold_ceil) {
+      if (pending > 0.0) {
         const double hold = (double)start + ((pending - 0.1) * (double)line_len);
         hold_floor = (long long)floor(hold);
         hold_ceil = (long long)ceil(hold);
         pending = -1.0;
       }
-    }
-    if (kept) {
-      keep_mask |= 1u << k;
-      types |= (unsigned long long)type << (2 * k);
-      cnt++;
+      keep(bit, type);
       cur = type;
     }
     if (done && vsync_seen) break;
   }
-  return WarpAttempt{done && cnt > 0, cnt, cur, keep_mask, types};
+  r.cnt = __popc(r.keep);
+  r.last = cur;
+  r.ok = done && r.cnt > 0;
+  return r;
 }
 
 // Block-wide sum of a long long (kLT threads); every thread gets the total.
@@ -652,7 +714,7 @@ __device__ int validate(const LineLocArgs& a, FieldSmem& sm, int n, VList& v) {
       const int o = p + __popc(r.keep & ((1u << lane) - 1u));
       v.s[o] = sm.ps[i - 2 + lane];
       v.l[o] = sm.pl[i - 2 + lane];
-      v.tg[o] = (unsigned char)((r.types >> (2 * lane)) & 3u);
+      v.tg[o] = (unsigned char)(((r.type0 >> lane) & 1u) | (((r.type1 >> lane) & 1u) << 1));
     }
   }
   __syncthreads();
@@ -1100,6 +1162,12 @@ __device__ const double* sorted_starts(FieldSmem& sm, const VList& v) {
         for (int q = 0; q < nruns; q++) {
           if (q == r) continue;
           int b = runs[q], e = runs[q + 1];  // entries of run q below x (at most x for an earlier run)
+          // most runs lie wholly before or after x: two reads settle them
+          if (v.s[e - 1] < x) {
+            rank += e - b;
+            continue;
+          }
+          if (v.s[b] > x) continue;
           while (b < e) {
             const int mid = (b + e) >> 1;
             const bool below = q < r ? v.s[mid] <= x : v.s[mid] < x;
@@ -1275,10 +1343,15 @@ __global__ void __launch_bounds__(kLT, 1) prepare_kernel(const __grid_constant__
   const int f = blockIdx.x, t = threadIdx.x;
   if (f >= a.win->fields) return;
   phase_clock(a, f, 0);
-  const int n = min(max(a.pn[f], 0), kMaxPulses);
-  for (int i = t; i < n; i += kLT) {
-    sm.ps[i] = a.ps[(size_t)f * kMaxPulses + i];
-    sm.pl[i] = a.pl[(size_t)f * kMaxPulses + i];
+  int n;
+  if (a.pulses_from_edges) {
+    n = window_pulses(a, f, sm.ps, sm.pl);
+  } else {
+    n = min(max(a.pn[f], 0), kMaxPulses);
+    for (int i = t; i < n; i += kLT) {
+      sm.ps[i] = a.ps[(size_t)f * kMaxPulses + i];
+      sm.pl[i] = a.pl[(size_t)f * kMaxPulses + i];
+    }
   }
   __syncthreads();
   phase_clock(a, f, 1);
@@ -1383,6 +1456,8 @@ __global__ void __launch_bounds__(kLT, 1) finish_kernel(const __grid_constant__ 
   __shared__ FieldPrep preps[kPrepBatch];
   __shared__ long long readlocs[kPrepBatch];
   __shared__ unsigned char fallback[kPrepBatch];
+  __shared__ unsigned stands_s[2];
+  static_assert(kPrepBatch == 64, "a 64-bit mask of the batch");
   __shared__ int fit_j, fit_first;
   __shared__ double prev_off_s, prev_loc_s, prev_diff_s;
   const int t = threadIdx.x;
@@ -1442,6 +1517,16 @@ __global__ void __launch_bounds__(kLT, 1) finish_kernel(const __grid_constant__ 
       fallback[i] = 0;
     }
     __syncthreads();
+    // bit j: field b0 + j's speculative anchor stands behind a field anchored past its window's start
+    bool ok = false;
+    if (t < nb) {
+      const FieldPrep& p = preps[t];
+      ok = p.vn > 0 && p.mll > 0.0 && !p.exact && p.spec_first >= 0 && p.spec.loc > 0.0;
+    }
+    const unsigned okm = __ballot_sync(0xffffffffu, ok);
+    if (t < 64 && (t & 31) == 0) stands_s[t >> 5] = okm;
+    __syncthreads();
+    const unsigned long long stands = (unsigned long long)stands_s[0] | ((unsigned long long)stands_s[1] << 32);
     int j = 0;
     while (j < nb) {
       if (t == 0) {
@@ -1449,6 +1534,24 @@ __global__ void __launch_bounds__(kLT, 1) finish_kernel(const __grid_constant__ 
           const int f = b0 + j;
           const FieldPrep& p = preps[j];
           const long long readloc = readlocs[j];
+          // A run of fields whose own votes fix their order and whose
+          // speculative anchors lie past their windows' starts stands as a
+          // whole once the field before it anchored there too: the last one's
+          // state is all that the walk carries on.  (Field by field the walk
+          // took 0.4 us a field, 17 of 29 us for 40 fields.)
+          const unsigned long long ahead = ~stands >> j;
+          const int run = ahead ? __ffsll((long long)ahead) - 1 : nb - j;
+          if (run > 0 && st.prev_first_hsync_loc > 0.0) {
+            for (int i = j; i < j + run; i++) a.is_first[b0 + i] = preps[i].spec_first;
+            const int l = j + run - 1;
+            if (run > 1) {
+              st.prev_first_hsync_readloc = readlocs[l - 1];
+              st.prev_first_hsync_loc = preps[l - 1].spec.loc;
+            }
+            anchored(b0 + l, readlocs[l], preps[l].spec_first != 0, preps[l].spec, preps[l].mll, true, 0.0);
+            j = l;
+            continue;
+          }
           if (!(p.vn > 0 && p.mll > 0.0)) {
             a.is_first[f] = st.prev_first_field >= 0 ? (1 - st.prev_first_field) : 1;
             fallback[j] = 1;
@@ -1814,6 +1917,7 @@ cudaError_t pulses_launch(const S& src, int portions, int max_fields, cudaStream
   return launch_chained(pulses_kernel<S>, dim3(max_fields, 1, portions), dim3(kLT), 0, st, src);
 }
 
+// With pulses_from_edges the per-field pass forms its own pulses.
 template <class S>
 cudaError_t lines_launch(const S& src, bool single_pass, int portions, int max_fields, cudaStream_t st) {
   if (max_fields <= 0) return cudaSuccess;

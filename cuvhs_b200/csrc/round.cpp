@@ -151,6 +151,7 @@ bool Context::decode_round(std::vector<Portion>& ps, const RoundPlan& next_plan)
     e.cap = (int)std::min<size_t>((size_t)p.num_fields * eps, INT_MAX / 2);
     em.a[j] = e;
     LineLocArgs la = lineloc_args(p.T, p.num_fields, (long long)p.raw_offset);
+    la.pulses_from_edges = single_pass ? 0 : 1;
     la.fall = e.fall;
     la.rise = e.rise;
     la.counts = e.counts;
@@ -211,19 +212,12 @@ bool Context::decode_round(std::vector<Portion>& ps, const RoundPlan& next_plan)
   // ---- edges, field windows and line locations on the line stream; the
   // guard after the edges; the pre-band-pass after the windows
   cudaStreamWaitEvent(lstream, ev_k1b, 0);
-  auto windows_and_lines = [&](bool from_bits) {
+  auto windows_and_lines = [&](bool again) {
     cudaMemsetAsync(d_counts, 0, (size_t)4 * L * sizeof(int), lstream);
     cudaEvent_t ev_;
     begin_stage_on(kStageEdges, ev_, lstream);
-    if (from_bits) {
-      launch_edges_bits_many(em, L, (long long)max_T * spp, lstream);
-    } else {
-      const float thr_rel = (float)(fmt.pulse_threshold_hz - fmt.ire0);
-      for (int j = 0; j < L; j++)
-        launch_edges(dm.a[j].sync, em.a[j].total, thr_rel, em.a[j].fall, em.a[j].rise, em.a[j].counts, em.a[j].cap,
-                     em.a[j].blk, d_edge_mask, lstream);
-    }
-    end_stage_on(kStageEdges, ev_, lstream, 3);
+    const int kernels = launch_edges_bits_many(em, L, (long long)max_T * spp, lstream);
+    end_stage_on(kStageEdges, ev_, lstream, kernels);
     cudaEventRecord(ev_edges, lstream);
     begin_stage_on(kStageWindows, ev_, lstream);
     launch_field_windows_many(lm, L, lstream);
@@ -233,15 +227,15 @@ bool Context::decode_round(std::vector<Portion>& ps, const RoundPlan& next_plan)
     cudaMemcpyAsync(hp_win, d_win, (size_t)L * sizeof(WindowInfo), cudaMemcpyDeviceToHost, xstream);
     cudaMemcpyAsync(hp_offs, d_offs, (size_t)slots * sizeof(long long), cudaMemcpyDeviceToHost, xstream);
     cudaEventRecord(ev_winhost, xstream);
-    cudaMemcpyAsync(from_bits ? d_lls_save : d_lls, from_bits ? d_lls : d_lls_save, (size_t)L * sizeof(LineLocState),
+    cudaMemcpyAsync(again ? d_lls : d_lls_save, again ? d_lls_save : d_lls, (size_t)L * sizeof(LineLocState),
                     cudaMemcpyDeviceToDevice, lstream);
     begin_stage_on(kStageLines, ev_, lstream);
-    launch_field_pulses_many(lm, L, max_nf, lstream);
+    if (single_pass) launch_field_pulses_many(lm, L, max_nf, lstream);
     launch_line_locations_many(lm, L, max_nf, lstream);
-    end_stage_on(kStageLines, ev_, lstream, single_pass ? 2 : 3);
+    end_stage_on(kStageLines, ev_, lstream, 2);
     cudaEventRecord(ev_ll, lstream);
   };
-  windows_and_lines(true);
+  windows_and_lines(false);
   {
     cudaStreamWaitEvent(gstream, ev_edges, 0);
     cudaMemsetAsync(d_guard_flips, 0, (size_t)L * sizeof(int), gstream);
@@ -278,7 +272,7 @@ bool Context::decode_round(std::vector<Portion>& ps, const RoundPlan& next_plan)
   }
   if (flips > 0) {
     cudaStreamWaitEvent(lstream, ev_guard, 0);
-    windows_and_lines(false);
+    windows_and_lines(true);
     if (cudaEventSynchronize(ev_winhost) != cudaSuccess) return check_cuda("round windows");
   }
   host_phase(kHostWindowsWait, t_host);
