@@ -150,9 +150,9 @@ struct DemodArgs {
   const float2* gb;
   const float2* tw_a;
   const float2* tw_b;
-  // The inverse transforms read their own copies of the twiddle tables, so the
-  // compiler cannot merge the two transforms' twiddle loads and keep them all
-  // live at once.
+  // The inverse transforms' twiddles: the same tables through pointers of
+  // their own, so that the compiler cannot merge the two transforms' loads and
+  // keep them all live at once (copies of the tables were twice what L1 holds).
   const float2* tw_a_inv;
   const float2* tw_b_inv;
   int a_pos, a_out, b_pos, b_out;
@@ -280,7 +280,7 @@ struct ChromaArgs {
   const double* ll;
   long long total;  // P * spp
   const int* track;  // per field
-  double het_scale;
+  const float* het;  // [2 tracks][out_h][out_w] heterodyne carrier (launch_het_table)
   int fsc_bin, bw_bins, burst_start, burst_len;
   int line_fft;      // per-line transform size (1024 or 2048)
   int out_w, out_h, lines_per_frame;
@@ -290,6 +290,9 @@ struct ChromaArgs {
   double* metric;    // per field burst cancellation metric
   const double* col_frac;  // [out_w]: (double)col / (double)out_w
 };
+// The heterodyne carrier of every output pixel for both tracks: it depends on
+// the row and column alone (chroma_decode.cu:75-157).
+void launch_het_table(float* het, double het_scale, int out_h, int out_w, cudaStream_t st);
 void launch_chroma_prefilter(const ChromaArgs& a, cudaStream_t st);
 // Lines [field0*out_h, (field0+nfields)*out_h) of the chunk.
 void launch_chroma_lines(const ChromaArgs& a, int field0, int nfields, bool write_output, cudaStream_t st);

@@ -15,6 +15,7 @@
 
 #include "chain.cuh"
 #include "cuvhs_internal.h"
+#include "numeric.cuh"
 #include "raw_input.cuh"
 #include "reg_fft.cuh"
 
@@ -31,23 +32,21 @@ namespace {
 constexpr int kElemsC = 16;
 constexpr int kThreadsC = Design::kNc / kElemsC;
 // Line kernel geometry: a line pair (two lines in one complex transform) per
-// group of line_tp threads with a padded N-point buffer (NTSC 1024, PAL 2048
-// points), line_pairs groups per CTA.  NTSC pairs take two warps, so each
-// thread holds one radix-16 butterfly per pass and the kernel fits 64
-// registers (32 warps per SM to cover the gathers' latency).
+// group of N/16 threads (NTSC 1024 points, 64 threads; PAL 2048, 128), so that
+// each thread holds one radix-16 butterfly per pass and the kernel fits 64
+// registers: 128-thread CTAs of two pairs or one, eight to an SM, to cover the
+// gathers' latency.  (A PAL pair on one warp took 254 registers: 135 us for 16
+// fields at 40 MHz.)
 template <int N>
-__host__ __device__ constexpr int line_tp() { return N <= 1024 ? 64 : 32; }
+__host__ __device__ constexpr int line_tp() { return N / 16; }
+constexpr int kLineThreads = 128;
 template <int N>
-__host__ __device__ constexpr int line_pairs() { return 2; }  // at most 4 (the two-warp barriers)
-template <int N>
-__host__ __device__ constexpr int line_threads() { return line_tp<N>() * line_pairs<N>(); }
-template <int N>
-__host__ __device__ constexpr int line_min_ctas() { return N <= 1024 ? 8 : 1; }
+__host__ __device__ constexpr int line_pairs() { return kLineThreads / line_tp<N>(); }  // 2 or 1
 
 // Barrier of one line pair's threads (the transform's barrier).
 template <int TP>
 __device__ __forceinline__ void pair_sync() {
-  static_assert(TP == 32 || TP == 64, "one or two warps per line pair");
+  static_assert(TP == 64 || TP == kLineThreads, "two warps of a CTA on a named barrier, or the whole CTA");
   fft_sync<TP>();
 }
 
@@ -104,13 +103,29 @@ __global__ void __launch_bounds__(kThreadsC, 1) prefilter_kernel(const __grid_co
   }
 }
 
+// The heterodyne carrier, a thread per pixel and track: phase in FP64 turns,
+// reduced before the FP32 cosine, plus the track's quarter turn per line.
+// Once per context: evaluated per pixel by every pass it was a third of the
+// line kernel's instructions, among them four of its six conversions a sample.
+constexpr int kHetThreads = 256;
+__global__ void __launch_bounds__(kHetThreads) het_table_kernel(float* het, double het_scale, int out_h, int out_w) {
+  const int p = blockIdx.x * kHetThreads + threadIdx.x;
+  if (p >= out_h * out_w) return;
+  const double u = het_scale * (double)p;
+  const float fr = (float)(u - floor(u));
+  for (int track = 0; track < 2; track++) {
+    const int rot = track ? 1 : 3;
+    const float lpf = 0.5f * (float)(((p / out_w) * rot) & 3);  // the rotation in half turns
+    het[(size_t)track * out_h * out_w + p] = -cospif(2.0f * fr + lpf);
+  }
+}
+
 // Per-line constants of the heterodyne resampler: the line's start and length
-// (chunk samples), its first output index and the track's quarter-turn
-// carrier rotation.  ok is false for lines past the line-location table.
+// (chunk samples) and its row of the carrier table.  ok is false for lines
+// past the line-location table.
 struct HetLine {
   double a0, span;
-  int ubase;  // row * out_w
-  float lpf;  // 0.5 * ((row * rot) & 3): the rotation in half turns
+  const float* het;
   bool ok;
 };
 
@@ -126,9 +141,7 @@ __device__ __forceinline__ HetLine het_line(const ChromaArgs& a, int gl) {
     L.a0 = a0;
     L.span = a1 - a0;
   }
-  const int rot = a.track[field] ? 1 : 3;
-  L.lpf = 0.5f * (float)((row * rot) & 3);
-  L.ubase = row * a.out_w;
+  L.het = a.het + ((size_t)(a.track[field] ? a.out_h : 0) + row) * a.out_w;
   return L;
 }
 
@@ -139,31 +152,27 @@ __device__ __forceinline__ HetLine het_line(const ChromaArgs& a, int gl) {
 __device__ __forceinline__ float het_at(const ChromaArgs& a, const HetLine& L, double frac, int c) {
   const double coord = L.a0 + frac * L.span;
   const int ci = (int)coord;
-  const bool ok = L.ok && ci >= 1 && (long long)ci + 2 < a.total;
+  const bool ok = L.ok && (unsigned)ci - 1u < tap_range(a.total);
   const int cl = ok ? ci : 1;
-  const float x = (float)(coord - (double)ci);
-  const float p0 = __ldg(&a.pre[cl - 1]), p1 = __ldg(&a.pre[cl]);
-  const float p2 = __ldg(&a.pre[cl + 1]), p3 = __ldg(&a.pre[cl + 2]);
+  const float x = (float)(coord - int_to_double(ci));
+  const float* p = a.pre + (cl - 1);
+  const float p0 = __ldg(p), p1 = __ldg(p + 1), p2 = __ldg(p + 2), p3 = __ldg(p + 3);
+  const float het = __ldg(L.het + c);
   const float c1 = p2 - p0;
   const float c2 = 2.0f * p0 - 5.0f * p1 + 4.0f * p2 - p3;
   const float c3 = 3.0f * (p1 - p2) + p3 - p0;
   const float v = p1 + 0.5f * x * (c1 + x * (c2 + x * c3));
-  // carrier phase in FP64 turns, reduced before the FP32 cosine
-  const double u = a.het_scale * (double)(L.ubase + c);
-  const float fr = (float)(u - floor(u));
-  const float het = -cospif(2.0f * fr + L.lpf);
   return ok ? v * het : 0.0f;
 }
 
 // nlines < 0: every line of the capture's a.fields fields (a batched round).
 template <int N, class Src>
-__global__ void __launch_bounds__(line_threads<N>(), line_min_ctas<N>())
+__global__ void __launch_bounds__(kLineThreads, 8)
     lines_kernel(const __grid_constant__ Src src, int line0, int nlines, int write_output) {
   const ChromaArgs& a = src.get();
   if (nlines < 0) nlines = a.fields * a.out_h;
   chain_wait();
   constexpr int TP = line_tp<N>(), P = line_pairs<N>();
-  static_assert(TP == 32 || P <= 4, "two-warp pairs use named barriers 1..4");
   __shared__ float2 sm_all[P][fft_pad(N)];
   __shared__ float acc_sh[P][2];
   const int g = threadIdx.x / TP, tid = threadIdx.x % TP, lane = threadIdx.x & 31;
@@ -176,41 +185,45 @@ __global__ void __launch_bounds__(line_threads<N>(), line_min_ctas<N>())
   HetLine B = A;
   if (has_b) B = het_line(a, line0 + lb);
   B.ok = B.ok && has_b;
-  // the gather is latency bound: unrolled so that several columns' loads are
-  // in flight (the FFT below sets the register budget, not this loop)
-#pragma unroll 4
-  for (int c = tid; c < N; c += TP) {
-    float va = 0.0f, vb = 0.0f;
+  // column tid + TP*q of both lines in slot q (the transform's layout)
+  float2 v[16];
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int c = tid + TP * q;
+    v[q] = make_float2(0.0f, 0.0f);
     if (c < a.out_w) {
       const double frac = __ldg(&a.col_frac[c]);
-      va = het_at(a, A, frac, c);
-      vb = het_at(a, B, frac, c);
+      v[q] = make_float2(het_at(a, A, frac, c), het_at(a, B, frac, c));
     }
-    sm[pidx(c)] = make_float2(va, vb);
   }
-  pair_sync<TP>();
-  smem_fft<N, TP, false>(sm, a.tw_line, tid);
+  RegFFT<N>::run<false>(v, sm, a.tw_line, tid);
+  // the band fsc +/- bw and its mirror lie in slots 3, 4, 11 and 12 (fsc is
+  // a quarter of the output rate, bw less than a sixteenth)
   const int lo = a.fsc_bin - a.bw_bins, hi = a.fsc_bin + a.bw_bins;
-  const float scale = 1.0f / (float)N;
-  for (int k = tid; k < N; k += TP) {
-    const int kk = k <= N / 2 ? k : N - k;
-    const float m = (kk >= lo && kk <= hi) ? scale : 0.0f;
-    const float2 x = sm[pidx(k)];
-    sm[pidx(k)] = make_float2(x.x * m, x.y * m);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int q = i < 2 ? 3 + i : 9 + i;
+    const int k = tid + TP * q, kk = k <= N / 2 ? k : N - k;
+    const float m = (kk >= lo && kk <= hi) ? 1.0f / (float)N : 0.0f;
+    v[q] = make_float2(v[q].x * m, v[q].y * m);
   }
-  pair_sync<TP>();
-  smem_fft<N, TP, true>(sm, a.tw_line_inv, opaque_index(tid));
+  RegFFT<N>::run_band<true>(v, sm, a.tw_line_inv, opaque_index(tid));
   // burst RMS per line -> ACC gain, summed by the pair's first warp in a
-  // fixed order (lane sums i = lane, lane + 32, ..., then a butterfly)
+  // fixed order (lane sums i = lane, lane + 32, ..., then a butterfly); the
+  // burst lies in the first two slots
+  pair_sync<TP>();  // the last pass's reads
+  sm[tid] = v[0];
+  sm[tid + TP] = v[1];
+  pair_sync<TP>();
   if (tid < 32) {
     const int bl = a.burst_len;
     float ssa = 0.0f, ssb = 0.0f;
     for (int i = lane; i < bl; i += 32) {
-      const float2 v = sm[pidx(a.burst_start + i)];
-      ssa += v.x * v.x;
-      ssb += v.y * v.y;
-      a.burst[(size_t)(line0 + la) * bl + i] = v.x;
-      if (has_b) a.burst[(size_t)(line0 + lb) * bl + i] = v.y;
+      const float2 x = sm[a.burst_start + i];
+      ssa += x.x * x.x;
+      ssb += x.y * x.y;
+      a.burst[(size_t)(line0 + la) * bl + i] = x.x;
+      if (has_b) a.burst[(size_t)(line0 + lb) * bl + i] = x.y;
     }
     for (int off = 16; off > 0; off >>= 1) {
       ssa += __shfl_xor_sync(0xffffffffu, ssa, off);
@@ -226,16 +239,36 @@ __global__ void __launch_bounds__(line_threads<N>(), line_min_ctas<N>())
   pair_sync<TP>();
   const float acc_a = acc_sh[g][0], acc_b = acc_sh[g][1];
   uint16_t* oa = a.chroma + (size_t)(line0 + la) * a.out_w;
-  uint16_t* ob = a.chroma + (size_t)(line0 + lb) * a.out_w;
-  for (int c = tid; c < a.out_w; c += TP) {
-    const float2 v = sm[pidx(c)];
-    const float xa = fminf(fmaxf(v.x * acc_a + 32768.0f, 0.0f), 65535.0f);
-    oa[c] = (uint16_t)(xa + 0.5f);
-    if (has_b) {
-      const float xb = fminf(fmaxf(v.y * acc_b + 32768.0f, 0.0f), 65535.0f);
-      ob[c] = (uint16_t)(xb + 0.5f);
-    }
+  uint16_t* ob = oa + a.out_w;
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int c = tid + TP * q;
+    if (c >= a.out_w) break;
+    oa[c] = trunc_u16(fminf(fmaxf(v[q].x * acc_a + 32768.0f, 0.0f), 65535.0f) + 0.5f);
+    if (has_b) ob[c] = trunc_u16(fminf(fmaxf(v[q].y * acc_b + 32768.0f, 0.0f), 65535.0f) + 0.5f);
   }
+}
+
+// Sum of |x + y| over two burst windows in sample order, the loads all issued
+// first (rows of BL floats start on 16-byte boundaries: BL is a multiple of 4).
+template <int BL>
+__device__ __forceinline__ double burst_pair_sum(const float* x, const float* y) {
+  static_assert(BL % 4 == 0, "16-byte rows");
+  float4 xv[BL / 4], yv[BL / 4];
+#pragma unroll
+  for (int q = 0; q < BL / 4; q++) {
+    xv[q] = __ldg(reinterpret_cast<const float4*>(x) + q);
+    yv[q] = __ldg(reinterpret_cast<const float4*>(y) + q);
+  }
+  double s = 0.0;
+#pragma unroll
+  for (int q = 0; q < BL / 4; q++) {
+    s += fabs((double)xv[q].x + (double)yv[q].x);
+    s += fabs((double)xv[q].y + (double)yv[q].y);
+    s += fabs((double)xv[q].z + (double)yv[q].z);
+    s += fabs((double)xv[q].w + (double)yv[q].w);
+  }
+  return s;
 }
 
 // One CTA per field: mean over line pairs (16+2p, 17+2p), p < (out_h - 33)/2,
@@ -263,21 +296,8 @@ __global__ void __launch_bounds__(kMetricThreads) metric_kernel(const __grid_con
     const float* x = a.burst + (size_t)line * bl;
     const float* y = x + bl;
     double s = 0.0;
-    if constexpr (BL > 0 && BL % 4 == 0) {
-      // rows start on 16-byte boundaries (BL floats per row)
-      float4 xv[BL / 4], yv[BL / 4];
-#pragma unroll
-      for (int q = 0; q < BL / 4; q++) {
-        xv[q] = __ldg(reinterpret_cast<const float4*>(x) + q);
-        yv[q] = __ldg(reinterpret_cast<const float4*>(y) + q);
-      }
-#pragma unroll
-      for (int q = 0; q < BL / 4; q++) {
-        s += fabs((double)xv[q].x + (double)yv[q].x);
-        s += fabs((double)xv[q].y + (double)yv[q].y);
-        s += fabs((double)xv[q].z + (double)yv[q].z);
-        s += fabs((double)xv[q].w + (double)yv[q].w);
-      }
+    if constexpr (BL > 0) {
+      s = burst_pair_sum<BL>(x, y);
     } else {
       for (int i = 0; i < bl; i++) s += fabs((double)x[i] + (double)y[i]);
     }
@@ -293,44 +313,49 @@ __global__ void __launch_bounds__(kMetricThreads) metric_kernel(const __grid_con
 }
 
 // The trial passes' burst metrics: per trial, pair means (one thread each,
-// the window summed in sample order) added in line order by one thread, the
-// host restatement's operations in its order, so the pick is the host's.
+// the window summed in sample order) added in line order by one thread (a
+// thread of a warp of its own per trial), the host restatement's operations in
+// its order, so the pick is the host's.  Latency bound: its loads one float at
+// a time and both sums on one thread took 10 us.
 constexpr int kPickThreads = 256;
+template <int BL>
 __global__ void __launch_bounds__(kPickThreads) track_pick_kernel(const TrackPickArgs a) {
   chain_wait();
   __shared__ double pair_mean[2][kPickThreads];
-  __shared__ int det;
-  const int skip = 16, bl = a.burst_len;
-  int npairs = 0;
-  for (int line = skip; line < a.out_h - skip - 1; line += 2) npairs++;
+  __shared__ double mean[2];
+  const int skip = 16;
+  int npairs = a.out_h - skip - 1 > skip ? (a.out_h - 2 * skip - 1 + 1) / 2 : 0;  // lines skip, skip + 2, ... < out_h - skip - 1
   npairs = min(npairs, kPickThreads);
   for (int k = threadIdx.x; k < 2 * npairs; k += kPickThreads) {
     const int t = k / npairs, p = k % npairs;
-    const float* x = (t ? a.burst1 : a.burst0) + (size_t)(skip + 2 * p) * bl;
-    const float* y = x + bl;
-    double s = 0.0;
-    for (int i = 0; i < bl; i++) s += fabs((double)x[i] + (double)y[i]);
-    pair_mean[t][p] = s / bl;
+    const float* x = (t ? a.burst1 : a.burst0) + (size_t)(skip + 2 * p) * BL;
+    pair_mean[t][p] = burst_pair_sum<BL>(x, x + BL) / BL;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double m[2];
-    for (int t = 0; t < 2; t++) {
-      double total = 0.0;
-      for (int p = 0; p < npairs; p++) total += pair_mean[t][p];
-      m[t] = npairs > 0 ? total / npairs : 1e9;
-    }
-    det = (m[1] < m[0]) ? 1 : 0;
-    *a.pick = det;
+  if (threadIdx.x == 0 || threadIdx.x == 32) {
+    const int t = threadIdx.x >> 5;
+    double total = 0.0;
+#pragma unroll 8
+    for (int p = 0; p < npairs; p++) total += pair_mean[t][p];
+    mean[t] = npairs > 0 ? total / npairs : 1e9;
   }
   __syncthreads();
+  const int det = (mean[1] < mean[0]) ? 1 : 0;
+  if (threadIdx.x == 0) *a.pick = det;
   for (int f = threadIdx.x; f < a.fields; f += kPickThreads) a.track[f] = (f & 1) ? (1 - det) : det;
 }
 
 }  // namespace
 
+void launch_het_table(float* het, double het_scale, int out_h, int out_w, cudaStream_t st) {
+  const int n = out_h * out_w;
+  het_table_kernel<<<(n + kHetThreads - 1) / kHetThreads, kHetThreads, 0, st>>>(het, het_scale, out_h, out_w);
+}
+
 void launch_track_pick(const TrackPickArgs& a, cudaStream_t st) {
-  launch_chained(track_pick_kernel, dim3(1), dim3(kPickThreads), 0, st, a);
+  // burst windows: 36 samples NTSC, 40 PAL
+  launch_chained(a.burst_len == 40 ? track_pick_kernel<40> : track_pick_kernel<36>, dim3(1), dim3(kPickThreads), 0, st,
+                 a);
 }
 
 namespace {
@@ -352,14 +377,14 @@ void lines_launch(const S& src, const ChromaArgs& a, int portions, int line0, in
                   bool write_output, cudaStream_t st) {
   if (max_lines <= 0) return;
   const int pairs = (max_lines + 1) / 2;
-  auto go = [&](auto kernel, int per_cta, int threads) {
+  auto go = [&](auto kernel, int per_cta) {
     // the largest shared-memory carveout, so that the register limit sets the CTAs per SM
     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    launch_chained(kernel, dim3((pairs + per_cta - 1) / per_cta, 1, portions), dim3(threads), 0, st, src, line0,
-                   nlines, write_output ? 1 : 0);
+    launch_chained(kernel, dim3((pairs + per_cta - 1) / per_cta, 1, portions), dim3(kLineThreads), 0, st, src,
+                   line0, nlines, write_output ? 1 : 0);
   };
-  if (a.line_fft == 2048) go(lines_kernel<2048, S>, line_pairs<2048>(), line_threads<2048>());
-  else go(lines_kernel<1024, S>, line_pairs<1024>(), line_threads<1024>());
+  if (a.line_fft == 2048) go(lines_kernel<2048, S>, line_pairs<2048>());
+  else go(lines_kernel<1024, S>, line_pairs<1024>());
 }
 
 template <class S>

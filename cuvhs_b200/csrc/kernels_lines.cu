@@ -7,10 +7,12 @@
 // the integer window truncations match.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "chain.cuh"
 #include "cuvhs_internal.h"
+#include "numeric.cuh"
 
 namespace cuvhs {
 namespace {
@@ -24,15 +26,14 @@ __device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync
 // A line's sync samples: the window the refinement reads is staged in shared
 // memory (one coalesced burst per warp instead of a dependent global load per
 // scan step); a position outside the staged range reads global memory, so the
-// result never depends on the staging.
+// result never depends on the staging.  Chunk positions fit 32 bits.
 struct SyncWindow {
   const float* g;   // the chunk's sync signal
   const float* sm;  // staged samples [lo, lo + n)
-  long long lo;
-  int n;
-  __device__ __forceinline__ float operator()(long long i) const {
-    const long long k = i - lo;
-    return (unsigned long long)k < (unsigned long long)n ? sm[k] : __ldg(g + i);
+  int lo, n;
+  __device__ __forceinline__ float operator()(int i) const {
+    const unsigned k = (unsigned)(i - lo);
+    return k < (unsigned)n ? sm[k] : __ldg(g + i);
   }
 };
 
@@ -49,29 +50,41 @@ __host__ __device__ inline int hsync_window(double us, double hw) {
   return n <= kHsyncWinMax ? n : 0;
 }
 
-// First sample pair (i-1, i) in [start, start+count) with prev >= target > cur;
-// returns the linearly interpolated crossing or -1.  The warp tests 32 pairs
-// per step and takes the lowest hit, so the result is the sequential scan's.
-__device__ double falling_cross(const SyncWindow& s, int start, int count, double target, long long total,
-                                int lane) {
+// First sample pair (i-1, i) in [start, start+count) that crosses target;
+// returns the linearly interpolated crossing or -1.  FALL: prev >= target >
+// cur; else prev < target <= cur (and nothing if the first sample lies above
+// it).  The warp tests 32 pairs per step and takes the lowest hit, so the
+// result is the sequential scan's.  A sample is FP32, so it lies at or above
+// the FP64 target exactly when it is at or above the first FP32 value there:
+// the scan compares in FP32 and only the hit is interpolated in FP64.
+template <bool FALL>
+__device__ double crossing(const SyncWindow& s, int start, int count, double target, long long total, int lane) {
   if (start < 0 || (long long)start + count > total || count < 2) return -1.0;
+  const float level = __double2float_ru(target);
+  if (!FALL && (double)s(start) > target) return -1.0;
   for (int base = start + 1; base < start + count; base += 32) {
     const int i = base + lane;
-    double p = 0.0, q = 0.0;
+    float p = 0.0f, q = 0.0f;
     bool hit = false;
     if (i < start + count) {
       p = s(i - 1);
       q = s(i);
-      hit = p >= target && q < target;
+      hit = FALL ? (p >= level && q < level) : (p < level && q >= level);
     }
     const unsigned m = __ballot_sync(kFull, hit);
     if (m) {
       const int src = __ffs(m) - 1;
       double r = 0.0;
       if (lane == src) {
-        const double a = p - target, b = q - target;
-        const double fr = (a - b != 0.0) ? (a / (a - b)) : 0.0;
-        r = (double)(i - 1) + fr;
+        if (FALL) {
+          const double a = (double)p - target, b = (double)q - target;
+          const double fr = (a - b != 0.0) ? (a / (a - b)) : 0.0;
+          r = (double)(i - 1) + fr;
+        } else {
+          const double a = target - (double)p, b = target - (double)q;
+          const double fr = (a + b != 0.0) ? (a / (a - b)) : 0.0;
+          r = (double)(i - 1) + fr;
+        }
       }
       return shfl_d(r, src);
     }
@@ -79,77 +92,43 @@ __device__ double falling_cross(const SyncWindow& s, int start, int count, doubl
   return -1.0;
 }
 
-__device__ double rising_cross(const SyncWindow& s, int start, int count, double target, long long total,
-                               int lane) {
-  if (start < 0 || (long long)start + count > total || count < 2) return -1.0;
-  if ((double)s(start) > target) return -1.0;
-  for (int base = start + 1; base < start + count; base += 32) {
-    const int i = base + lane;
-    double p = 0.0, q = 0.0;
-    bool hit = false;
-    if (i < start + count) {
-      p = s(i - 1);
-      q = s(i);
-      hit = p < target && q >= target;
-    }
-    const unsigned m = __ballot_sync(kFull, hit);
-    if (m) {
-      const int src = __ffs(m) - 1;
-      double r = 0.0;
-      if (lane == src) {
-        const double a = target - p, b = target - q;
-        const double fr = (a + b != 0.0) ? (a / (a - b)) : 0.0;
-        r = (double)(i - 1) + fr;
-      }
-      return shfl_d(r, src);
-    }
-  }
-  return -1.0;
-}
+// x or y: the larger one or the smaller one.
+__device__ __forceinline__ float keep(float x, float y, bool larger) { return ((x > y) != larger) ? y : x; }
 
-// One compare-exchange stage of a warp bitonic sort: element e (value x) and
-// element e ^ j (lane ^ j), ascending within blocks of k elements whose
-// index bit k is clear, descending in the others.
-__device__ __forceinline__ float bitonic_stage(float x, int e, int j, int k) {
-  const float y = __shfl_xor_sync(kFull, x, j);
-  const bool keep_min = ((e & k) == 0) == ((e & j) == 0);
-  return keep_min ? fminf(x, y) : fmaxf(x, y);
+// Ascending sort of one value per lane: bitonic merges whose first step meets
+// the mirrored partner (lane ^ (k - 1)), so that every step leaves the smaller
+// value in the lane whose bit is clear: five lane predicates serve all 15
+// steps, three instructions each (with the direction alternating by block, the
+// step's own predicate made it six).
+__device__ __forceinline__ float sort32(float x, int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32; k <<= 1) {
+    x = keep(x, __shfl_xor_sync(kFull, x, k - 1), (lane & (k >> 1)) != 0);
+#pragma unroll
+    for (int j = k >> 2; j > 0; j >>= 1) x = keep(x, __shfl_xor_sync(kFull, x, j), (lane & j) != 0);
+  }
+  return x;
 }
 
 // Order statistic n/2 of the window (the upper median for even n), n <= 64:
-// the window, padded with +inf, is sorted across the warp by a bitonic
-// network (32 elements, one per lane, when n <= 32; else 64, lane l holding
-// elements l and l + 32), and element n/2 is read from its lane.  Ties hold
+// the window, padded with +inf, is sorted across the warp (32 elements, one
+// per lane, when n <= 32; else two sorted halves and the merge of the half
+// that holds element n/2), and element n/2 is read from its lane.  Ties hold
 // equal values, so the result is the window's order statistic whichever
 // duplicate lands there.
 __device__ double window_median(const SyncWindow& s, int start, int count, long long total, int lane) {
   if (start < 0 || (long long)start + count > total || count <= 0) return 0.0;
   const int n = min(count, 64);
   const int mid = n / 2;
-  float x0 = lane < n ? s(start + lane) : INFINITY;
-  if (n <= 32) {
+  float x = sort32(lane < n ? s(start + lane) : INFINITY, lane);
+  if (n > 32) {
+    const float x1 = sort32(lane + 32 < n ? s(start + lane + 32) : INFINITY, lane);
+    const float y = __shfl_xor_sync(kFull, mid < 32 ? x1 : x, 31);  // the mirrored partner of either half
+    x = mid < 32 ? fminf(x, y) : fmaxf(x1, y);
 #pragma unroll
-    for (int k = 2; k <= 32; k <<= 1)
-#pragma unroll
-      for (int j = k >> 1; j > 0; j >>= 1) x0 = bitonic_stage(x0, lane, j, k);
-    return (double)__shfl_sync(kFull, x0, mid);
+    for (int j = 16; j > 0; j >>= 1) x = keep(x, __shfl_xor_sync(kFull, x, j), (lane & j) != 0);
   }
-  float x1 = lane + 32 < n ? s(start + lane + 32) : INFINITY;
-#pragma unroll
-  for (int k = 2; k <= 64; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j == 32) {  // partners in the same lane; k = 64 sorts ascending
-        const float lo = fminf(x0, x1), hi = fmaxf(x0, x1);
-        x0 = lo;
-        x1 = hi;
-      } else {
-        x0 = bitonic_stage(x0, lane, j, k);
-        x1 = bitonic_stage(x1, lane + 32, j, k);
-      }
-    }
-  }
-  return (double)__shfl_sync(kFull, mid < 32 ? x0 : x1, mid & 31);
+  return (double)__shfl_sync(kFull, x, mid & 31);
 }
 
 // One warp per line location (lines from the first active line to the end of
@@ -182,13 +161,13 @@ __global__ void __launch_bounds__(32 * kHsyncWarps) hsync_kernel(const __grid_co
       const float4* g4 = reinterpret_cast<const float4*>(a.sync + lo);
       for (int k = lane; k < n4; k += 32) reinterpret_cast<float4*>(w)[k] = __ldg(g4 + k);
       for (int k = 4 * n4 + lane; k < n; k += 32) w[k] = __ldg(a.sync + lo + k);
-      s.lo = lo;
+      s.lo = (int)lo;
       s.n = n;
     }
     __syncwarp();
   }
   // leading (falling) edge
-  const double zc = falling_cross(s, (int)(orig - ou), ou * 2, thr, a.total, lane);
+  const double zc = crossing<true>(s, (int)(orig - ou), ou * 2, thr, a.total, lane);
   double left = -1.0;
   if (zc >= 0.0) {
     const int zi = (int)(zc + 0.5);
@@ -196,20 +175,20 @@ __global__ void __launch_bounds__(32 * kHsyncWarps) hsync_kernel(const __grid_co
     const double porch_lv = window_median(s, zi + (int)(8.0 * us), (int)(1.0 * us), a.total, lane);
     if (porch_lv > sync_lv) {
       const double mid = (sync_lv + porch_lv) / 2.0;
-      const double zc2 = falling_cross(s, (int)(orig - ou * 2), (int)(us * 4), mid, a.total, lane);
+      const double zc2 = crossing<true>(s, (int)(orig - ou * 2), (int)(us * 4), mid, a.total, lane);
       if (zc2 >= 0.0 && fabs(zc2 - zc) <= us * 0.5) left = zc2;
     }
   }
   // trailing (rising) edge
   double right = -1.0;
-  const double rx = rising_cross(s, (int)(orig + hw - us), (int)(hw * 2), thr, a.total, lane);
+  const double rx = crossing<false>(s, (int)(orig + hw - us), (int)(hw * 2), thr, a.total, lane);
   if (rx >= 0.0) {
     const int zfi = (int)(rx - hw + 0.5);
     const double rs = window_median(s, zfi + (int)(1.0 * us), (int)(1.5 * us), a.total, lane);
     const double rp = window_median(s, zfi + (int)(hw + 1.0 * us), (int)(1.0 * us), a.total, lane);
     if (rp > rs) {
       const double rmid = (rs + rp) / 2.0;
-      const double zc2r = rising_cross(s, (int)(orig + hw - us), (int)(hw * 2), rmid, a.total, lane);
+      const double zc2r = crossing<false>(s, (int)(orig + hw - us), (int)(hw * 2), rmid, a.total, lane);
       if (zc2r >= 0.0 && fabs(zc2r - rx) <= us * 0.5) {
         const double cand = rx - hw + a.right_edge_offset;
         const double ref = (left >= 0.0) ? left : orig;
@@ -231,7 +210,17 @@ __global__ void __launch_bounds__(32 * kHsyncWarps) hsync_kernel(const __grid_co
 // to three output columns), then every Catmull-Rom tap reads shared memory.
 // A row whose window would not fit (line locations of a lost signal) reads
 // global memory directly, with the same arithmetic.
-constexpr int kLumaWindow = 4096;  // staged samples per row (a line is 1780 at 28 MHz, 2560 at 40 MHz PAL)
+//
+// Bound by instruction issue (66-71% of cycles; DRAM a third of its rate), then
+// by a row's chain of line starts, window and pixels: constant offsets from one
+// address a thread, one range test a pixel and no conversions that a bit
+// pattern replaces.
+constexpr int kLumaWindowMax = 4096;
+constexpr int kLumaColumns = (1135 + kLumaThreads - 1) / kLumaThreads;  // pixels a thread, the widest line (PAL)
+// Samples staged per row: a line and 6%, with room for the taps.
+inline int luma_window(double one_us) {
+  return std::min(kLumaWindowMax, ((int)(one_us * 64.0 * 1.06) + 32 + 31) & ~31);
+}
 
 __device__ __forceinline__ uint16_t luma_pixel(const LineArgs& a, float p0, float p1, float p2, float p3, float x,
                                                bool ok) {
@@ -241,18 +230,18 @@ __device__ __forceinline__ uint16_t luma_pixel(const LineArgs& a, float p0, floa
   const float hz = p1 + 0.5f * x * (c1 + x * (c2 + x * c3));
   float v = hz * a.luma_gain + a.luma_offset;
   v = fminf(fmaxf(v, 0.0f), 65535.0f);
-  return ok ? (uint16_t)(v + 0.5f) : a.oob_value;
+  return ok ? trunc_u16(v + 0.5f) : a.oob_value;
 }
 
 template <class Src>
-__global__ void __launch_bounds__(kLumaThreads) luma_kernel(const __grid_constant__ Src src) {
+__global__ void __launch_bounds__(kLumaThreads, 12) luma_kernel(const __grid_constant__ Src src, int window) {
   const LineArgs& a = src.get();
   const int W = a.out_w, H = a.out_h;
   const int grow = blockIdx.x;  // field * H + row
   const int field = grow / H, row = grow % H;
   if (field >= a.fields) return;  // whole CTA: a batched capture with fewer fields
   chain_wait();
-  __shared__ __align__(16) float win[kLumaWindow];
+  extern __shared__ __align__(16) float win[];
   uint16_t* out = a.luma + (size_t)grow * W;
   if (row + 1 >= a.lines_per_frame) {
     for (int col = threadIdx.x; col < W; col += kLumaThreads) out[col] = a.oob_value;
@@ -266,7 +255,7 @@ __global__ void __launch_bounds__(kLumaThreads) luma_kernel(const __grid_constan
   // may round a few ulp past either one, so the window reaches one more
   // sample each way)
   const double cmin = fmin(a0, a1), cmax = fmax(a0, a1);
-  bool staged = cmin >= -4.0 && cmax < (double)a.total && cmax - cmin < (double)(kLumaWindow - 16);
+  bool staged = cmin >= -4.0 && cmax < (double)a.total && cmax - cmin < (double)(window - 16);
   long long lo = 0;
   int n = 0;
   if (staged) {
@@ -274,7 +263,7 @@ __global__ void __launch_bounds__(kLumaThreads) luma_kernel(const __grid_constan
     if (lo < 0) lo = 0;
     const long long hi = min((long long)floor(cmax) + 4, a.total);
     n = (int)(hi - lo);
-    staged = n > 0 && n <= kLumaWindow;
+    staged = n > 0 && n <= window;
   }
   if (staged) {
     const float* src = a.video + lo;
@@ -284,14 +273,19 @@ __global__ void __launch_bounds__(kLumaThreads) luma_kernel(const __grid_constan
       reinterpret_cast<float4*>(win)[i] = __ldg(reinterpret_cast<const float4*>(src) + i);
     for (int i = 4 * n4 + threadIdx.x; i < n; i += kLumaThreads) win[i] = __ldg(&src[i]);
     __syncthreads();
-#pragma unroll 4
-    for (int col = threadIdx.x; col < W; col += kLumaThreads) {
-      const double coord = a0 + __ldg(&a.col_frac[col]) * span;
+    const double* frac = a.col_frac + threadIdx.x;
+    uint16_t* o = out + threadIdx.x;
+    const unsigned inside = tap_range(a.total);
+    const int shift = 1 - (int)lo;  // tap ci - 1 of an in-range column at win[ci - 1 - lo]
+#pragma unroll
+    for (int i = 0; i < kLumaColumns; i++) {
+      if (threadIdx.x + i * kLumaThreads >= W) break;
+      const double coord = a0 + __ldg(frac + i * kLumaThreads) * span;
       const int ci = (int)coord;
-      const bool ok = ci >= 1 && (long long)ci + 2 < a.total;
-      const int k = ok ? (int)((long long)ci - lo) : 1;  // in-range taps lie in the window
-      const float x = (float)(coord - (double)ci);
-      out[col] = luma_pixel(a, win[k - 1], win[k], win[k + 1], win[k + 2], x, ok);
+      const bool ok = (unsigned)ci - 1u < inside;
+      const float* p = win + (ok ? ci - 2 + shift : 0);
+      const float x = (float)(coord - int_to_double(ci));
+      o[i * kLumaThreads] = luma_pixel(a, p[0], p[1], p[2], p[3], x, ok);
     }
     return;
   }
@@ -304,7 +298,7 @@ __global__ void __launch_bounds__(kLumaThreads) luma_kernel(const __grid_constan
     const int ci = (int)coord;
     const bool ok = ci >= 1 && (long long)ci + 2 < a.total;
     const int cl = ok ? ci : 1;
-    const float x = (float)(coord - (double)ci);
+    const float x = (float)(coord - int_to_double(ci));
     out[col] = luma_pixel(a, __ldg(&a.video[cl - 1]), __ldg(&a.video[cl]), __ldg(&a.video[cl + 1]),
                           __ldg(&a.video[cl + 2]), x, ok);
   }
@@ -324,7 +318,8 @@ void launch_luma(const LineArgs& a, cudaStream_t st) {
   const int rows = a.fields * a.out_h;
   if (rows <= 0) return;
   using S = ArgsOne<LineArgs>;
-  launch_chained(luma_kernel<S>, dim3(rows), dim3(kLumaThreads), 0, st, S{a});
+  const int window = luma_window(a.one_us);
+  launch_chained(luma_kernel<S>, dim3(rows), dim3(kLumaThreads), window * sizeof(float), st, S{a}, window);
 }
 
 void launch_hsync_refine_many(const ArgsMany<LineArgs>& p, int portions, int max_fields, cudaStream_t st) {
@@ -338,7 +333,9 @@ void launch_hsync_refine_many(const ArgsMany<LineArgs>& p, int portions, int max
 void launch_luma_many(const ArgsMany<LineArgs>& p, int portions, int max_fields, cudaStream_t st) {
   const int rows = max_fields * p.a[0].out_h;
   if (rows <= 0 || portions <= 0) return;
-  launch_chained(luma_kernel<ArgsMany<LineArgs>>, dim3(rows, 1, portions), dim3(kLumaThreads), 0, st, p);
+  const int window = luma_window(p.a[0].one_us);
+  launch_chained(luma_kernel<ArgsMany<LineArgs>>, dim3(rows, 1, portions), dim3(kLumaThreads), window * sizeof(float),
+                 st, p, window);
 }
 
 }  // namespace cuvhs

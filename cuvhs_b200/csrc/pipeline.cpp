@@ -223,10 +223,10 @@ bool Context::alloc_buffers() {
   d_twb = A((float2*)nullptr, des.tw_b.size());
   d_twc = A((float2*)nullptr, des.tw_c.size());
   d_twl = A((float2*)nullptr, des.tw_line.size());
-  d_twa_inv = A((float2*)nullptr, des.tw_a.size());
-  d_twb_inv = A((float2*)nullptr, des.tw_b.size());
-  d_twc_inv = A((float2*)nullptr, des.tw_c.size());
-  d_twl_inv = A((float2*)nullptr, des.tw_line.size());
+  d_twa_inv = d_twa;
+  d_twb_inv = d_twb;
+  d_twc_inv = d_twc;
+  d_twl_inv = d_twl;
   d_win = A((WindowInfo*)nullptr, kMaxPortions);
   d_offs = A((long long*)nullptr, (size_t)batch + 1);
   d_cand = A((int*)nullptr, edge_alloc);
@@ -252,6 +252,7 @@ bool Context::alloc_buffers() {
   d_dbg_clk_ll = A((long long*)nullptr, (size_t)batch * kPhaseSlots);
   d_dbg_clk_guard = A((long long*)nullptr, (size_t)kGuardClockSamples * kPhaseSlots);
   d_col_frac = A((double*)nullptr, (size_t)fmt.output_line_len);
+  d_het = A((float*)nullptr, 2 * F);
   d_guard_g = A((double2*)nullptr, (size_t)Design::kGuardN);
   d_guard_tw = A((double2*)nullptr, (size_t)Design::kGuardN);
   d_hs64 = A((double*)nullptr, des.hs64.size());
@@ -453,10 +454,6 @@ bool Context::init(const cuvhs_config& c) {
   upload(d_twb, des.tw_b, stream);
   upload(d_twc, des.tw_c, stream);
   upload(d_twl, des.tw_line, stream);
-  upload(d_twa_inv, des.tw_a, stream);
-  upload(d_twb_inv, des.tw_b, stream);
-  upload(d_twc_inv, des.tw_c, stream);
-  upload(d_twl_inv, des.tw_line, stream);
   cudaMemcpyAsync(d_guard_g, des.guard_g.data(), des.guard_g.size() * sizeof(double), cudaMemcpyHostToDevice, stream);
   cudaMemcpyAsync(d_guard_tw, des.guard_tw.data(), des.guard_tw.size() * sizeof(double), cudaMemcpyHostToDevice,
                   stream);
@@ -469,6 +466,7 @@ bool Context::init(const cuvhs_config& c) {
   std::vector<double> col_frac(fmt.output_line_len);
   for (int c = 0; c < fmt.output_line_len; c++) col_frac[c] = (double)c / (double)fmt.output_line_len;
   upload(d_col_frac, col_frac, stream);
+  launch_het_table(d_het, des.het_scale, fmt.output_field_lines, fmt.output_line_len, stream);
   if (cudaStreamSynchronize(stream) != cudaSuccess) {
     err = std::string("upload failed: ") + cudaGetErrorString(cudaGetLastError());
     status = CUVHS_ERR_CUDA;
@@ -671,7 +669,7 @@ ChromaArgs Context::chroma_args(const uint8_t* raw, int n_read, const float* dc,
   ca.ll = d_ll;
   ca.total = 0;
   ca.track = d_track;
-  ca.het_scale = des.het_scale;
+  ca.het = d_het;
   ca.fsc_bin = des.fsc_bin;
   ca.bw_bins = des.bw_bins;
   ca.burst_start = fmt.burst_start;

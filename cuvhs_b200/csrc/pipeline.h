@@ -173,6 +173,7 @@ struct Context {
   int *d_do_count = nullptr, *d_do_lines = nullptr, *d_do_starts = nullptr, *d_do_ends = nullptr;
   unsigned char* d_do_cls = nullptr;
   double* d_col_frac = nullptr;
+  float* d_het = nullptr;  // heterodyne carrier per track, row and column
   // line location (kernels_linelocs.cu)
   WindowInfo* d_win = nullptr;
   long long* d_offs = nullptr;

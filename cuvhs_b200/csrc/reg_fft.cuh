@@ -1,8 +1,9 @@
-// Register-resident block FFT for one CTA of T = N/16 threads (sm_100a).
+// Register-resident block FFT for T = N/16 threads (sm_100a): a CTA, or for N =
+// 1024 a group of two warps.
 //
 // Thread t owns elements t + T*q, q = 0..15, of an N-point transform, both on
 // entry (natural-order input) and on exit (natural-order output): radix-16
-// passes (and one final radix 2/4 when N is not a power of 16) exchange data
+// passes (and one final radix 2/4/8 when N is not a power of 16) exchange data
 // through a padded shared buffer between passes, but the first
 // pass reads its inputs from registers and the last pass leaves its outputs in
 // registers.  Since the output layout equals the input layout, a forward
@@ -30,7 +31,7 @@ namespace cuvhs {
 
 template <int N>
 struct RegFFT {
-  static_assert(N == 4096 || N == 8192 || N == 16384, "three radix-16 passes and a last one of 1, 2 or 4");
+  static_assert(N >= 1024 && N <= 16384 && (N & (N - 1)) == 0, "two radix-16 passes or three, and a smaller last one");
   static constexpr int T = N / 16;
 
   // Padded location of slot 0 of thread t's (first) butterfly in the pass of
@@ -40,16 +41,17 @@ struct RegFFT {
   __device__ __forceinline__ static int place(int t) {
     const int lo = t & 15, mid = ((t >> 4) & 15) * T, hi = t >> 8;
     if constexpr (NS == 16) return pidx(t);
+    else if constexpr (N < 4096) return pidx(lo + (t >> 4) * T);
     else if constexpr (NS == 256) return pidx(hi * 16 + lo + mid);
     else return pidx(hi * (T / 16) + lo + mid);
   }
   template <int NS>
   __host__ __device__ static constexpr int slot_stride() {
-    return NS == 16 ? fft_pad(T) : (NS == 256 ? fft_pad(T / 16) : 17);
+    return NS == 16 ? fft_pad(T) : (NS == 256 && N >= 4096 ? fft_pad(T / 16) : 17);
   }
   template <int NS>
-  __host__ __device__ static constexpr int butterfly_stride() {  // the last pass of N > 4096 has several
-    return fft_pad((T / 256) * (T / 16));
+  __host__ __device__ static constexpr int butterfly_stride() {  // the last pass has several where N is no power of 16
+    return N < 4096 ? fft_pad((T / 16) * T) : fft_pad((T / 256) * (T / 16));
   }
 
   // One pass of radix R at span NS (> 1).  LAST leaves the results in v in the
@@ -79,7 +81,7 @@ struct RegFFT {
     } else {
 #pragma unroll
       for (int r = 0; r < R; r++) p[r * slot_stride<NS>()] = w[0][dft_slot<R>(r)];
-      __syncthreads();
+      fft_sync<T>();
     }
   }
 
@@ -115,13 +117,20 @@ struct RegFFT {
     after_first<INV>(v, s, tw, t);
   }
 
+  // run() of an input that is zero but for slots 3, 4, 11 and 12.
+  template <bool INV>
+  __device__ __forceinline__ static void run_band(float2 (&v)[16], float2* s, const float2* __restrict__ tw, int t) {
+    dft16_band<INV>(v);
+    after_first<INV>(v, s, tw, t);
+  }
+
   template <bool INV>
   __device__ __forceinline__ static void after_first(float2 (&v)[16], float2* s, const float2* __restrict__ tw,
                                                      int t) {
-    __syncthreads();
+    fft_sync<T>();
 #pragma unroll
     for (int r = 0; r < 16; r++) s[pidx(16 * t + r)] = v[dft_slot<16>(r)];
-    __syncthreads();
+    fft_sync<T>();
     rest<16, INV>(v, s, tw, t);
   }
 };

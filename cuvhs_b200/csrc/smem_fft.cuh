@@ -168,6 +168,26 @@ __device__ __forceinline__ void dft16_gains(float2* v, const float* g) {
   dft16_second<INV>(v);
 }
 
+// dft<16, INV> of an input that is zero but for v[3], v[4], v[11] and v[12]
+// (the others are not read): a band around a quarter of the sample rate and
+// its mirror image.
+template <bool INV>
+__device__ __forceinline__ void dft16_band(float2* v) {
+  // the dft4 over n1 of columns n2 = 0 and 3, for k1 = 0..3
+  const float2 s0 = cadd(v[4], v[12]), d0 = mul_mi<INV>(csub(v[4], v[12]));
+  const float2 s3 = cadd(v[3], v[11]), d3 = csub(v[3], v[11]);
+  const float2 a0[4] = {s0, d0, make_float2(-s0.x, -s0.y), make_float2(-d0.x, -d0.y)};
+  const float2 a3[4] = {s3, rot<16, 3, INV>(d3), rot<16, 6, INV>(s3), rot<16, 9, INV>(d3)};
+#pragma unroll
+  for (int k1 = 0; k1 < 4; k1++) {
+    const float2 m = mul_mi<INV>(a3[k1]);
+    v[4 * k1] = cadd(a0[k1], a3[k1]);
+    v[4 * k1 + 2] = csub(a0[k1], a3[k1]);
+    v[4 * k1 + 1] = csub(a0[k1], m);
+    v[4 * k1 + 3] = cadd(a0[k1], m);
+  }
+}
+
 // dft<16, INV> of an input whose upper half v[8..15] is zero (not read).
 template <bool INV>
 __device__ __forceinline__ void dft16_half(float2* v) {
