@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(kPickThreads) track_pick_kernel(const TrackPic
 #pragma unroll 8
     for (int p = 0; p < npairs; p++) total += pair_mean[t][p];
     mean[t] = npairs > 0 ? total / npairs : 1e9;
+    a.mean[t] = mean[t];
   }
   __syncthreads();
   const int det = (mean[1] < mean[0]) ? 1 : 0;

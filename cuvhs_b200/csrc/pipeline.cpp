@@ -211,6 +211,7 @@ bool Context::alloc_buffers() {
   d_trial = A((int*)nullptr, 2);
   d_burst_trial = A((float*)nullptr, (size_t)2 * fmt.output_field_lines * fmt.burst_len);
   d_pick = A((int*)nullptr, 1);
+  d_trial_mean = A((double*)nullptr, 2);
   d_do_count = A((int*)nullptr, batch);
   d_do_lines = A((int*)nullptr, (size_t)batch * kMaxDropouts);
   d_do_starts = A((int*)nullptr, (size_t)batch * kMaxDropouts);
@@ -282,12 +283,14 @@ bool Context::alloc_buffers() {
   hp_counts = H((int*)nullptr, 4);
   hp_win = H((WindowInfo*)nullptr, kMaxPortions);
   hp_lls = H((LineLocState*)nullptr, kMaxPortions);
+  hp_lls_fresh = H((LineLocState*)nullptr, 1);
   hp_offs = H((long long*)nullptr, (size_t)batch + 1);
   hp_is_first = H((int*)nullptr, batch);
   hp_guard = H((int*)nullptr, 2 * kMaxPortions);
   hp_track = H((int*)nullptr, batch);
   hp_trial = H((int*)nullptr, 2);
   hp_pick = H((int*)nullptr, 1);
+  hp_trial_mean = H((double*)nullptr, 2);
   hp_burst = H((float*)nullptr, (size_t)2 * fmt.output_field_lines * fmt.burst_len);
   {
     void* p = nullptr;
@@ -418,6 +421,7 @@ bool Context::init(const cuvhs_config& c) {
     }
     b = std::max(1, b / 2);
   }
+  *hp_lls_fresh = LineLocState();
   hp_trial[0] = 0;
   hp_trial[1] = 1;
   if (cudaMemcpy(d_trial, hp_trial, 2 * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -529,7 +533,7 @@ bool Context::wait_host_event(const char* where) {
 }
 
 void Context::reset_state() {
-  if (d_lls) write_lls(LineLocState());
+  lls_reset = true;  // the device copy follows with the next work that reads it
   chroma_valid = false;
   chroma_track = 0;
   chroma_threshold = 0.0;
@@ -559,15 +563,21 @@ double host_burst_metric(const float* b, int H, int bl) {
 double host_burst_phase(const float* b, int H, const Format& fmt) {
   const int skip = 16;
   const double PI = 3.14159265358979323846;
+  // the reference product's carrier, the same for every line
+  double cs[kMaxBurstLen], sn[kMaxBurstLen];
+  for (int i = 0; i < fmt.burst_len; i++) {
+    const double t = 2.0 * PI * fmt.fsc / fmt.output_rate * (double)(fmt.burst_start + i);
+    cs[i] = std::cos(t);
+    sn[i] = std::sin(t);
+  }
   double It = 0.0, Qt = 0.0;
   for (int line = skip; line < H - skip; line++) {
     const float* x = b + (size_t)line * fmt.burst_len;
     double I = 0.0, Q = 0.0;
     for (int i = 0; i < fmt.burst_len; i++) {
       const double v = x[i];
-      const double t = 2.0 * PI * fmt.fsc / fmt.output_rate * (double)(fmt.burst_start + i);
-      I += v * std::cos(t);
-      Q += v * std::sin(t);
+      I += v * cs[i];
+      Q += v * sn[i];
     }
     const double m = std::sqrt(I * I + Q * Q);
     if (m > 0.0) {
@@ -803,7 +813,16 @@ LineLocArgs Context::lineloc_args(int tiles, int num_fields, long long raw_offse
   return a;
 }
 
+// A reset that has not reached the device yet, on the stream whose work reads
+// the state next.
+void Context::settle_lls(cudaStream_t st) {
+  if (!lls_reset) return;
+  lls_reset = false;
+  cudaMemcpyAsync(d_lls, hp_lls_fresh, sizeof(LineLocState), cudaMemcpyHostToDevice, st);
+}
+
 bool Context::read_lls(LineLocState& st) {
+  settle_lls(lstream);
   if (cudaStreamSynchronize(stream) != cudaSuccess || cudaStreamSynchronize(lstream) != cudaSuccess ||
       cudaMemcpy(&st, d_lls, sizeof(LineLocState), cudaMemcpyDeviceToHost) != cudaSuccess)
     return check_cuda("line-location state");
@@ -811,6 +830,7 @@ bool Context::read_lls(LineLocState& st) {
 }
 
 bool Context::write_lls(const LineLocState& st) {
+  lls_reset = false;
   if (cudaStreamSynchronize(stream) != cudaSuccess || cudaStreamSynchronize(lstream) != cudaSuccess ||
       cudaMemcpy(d_lls, &st, sizeof(LineLocState), cudaMemcpyHostToDevice) != cudaSuccess)
     return check_cuda("line-location state");
@@ -848,13 +868,13 @@ bool Context::chroma_fields(ChromaArgs& ca, int P, const DropoutArgs* conceal, u
                       cudaMemcpyDeviceToHost, ostream);
     }
   };
-  auto chroma_pass = [&](int f0, int nf, bool write) {
+  auto chroma_pass = [&](int f0, int nf, bool write, bool metric) {
     cudaEvent_t ev_;
     begin_stage_on(kStageChromaLines, ev_, cs);
     launch_chroma_lines(ca, f0, nf, write, cs);
     end_stage_on(kStageChromaLines, ev_, cs);
     cudaEventRecord(ev_cpass, cs);  // the concealment needs the lines, not the metric
-    if (write) {
+    if (metric) {
       begin_stage_on(kStageBurstMetric, ev_, cs);
       launch_burst_metric(ca, f0, nf, cs);  // writes hp_metric through its mapping
       end_stage_on(kStageBurstMetric, ev_, cs);
@@ -864,9 +884,10 @@ bool Context::chroma_fields(ChromaArgs& ca, int P, const DropoutArgs* conceal, u
   double thr;
   const bool on_device = trial_on_device && !chroma_valid;
   const size_t nb_ = (size_t)H * fmt.burst_len;
+  // (the device pick forms the means in host_burst_metric's operations and order)
   auto detect = [&](int& det, double& th, int& cyc) {
-    const double m0 = host_burst_metric(hp_burst, H, fmt.burst_len),
-                 m1 = host_burst_metric(hp_burst + nb_, H, fmt.burst_len);
+    const double m0 = on_device ? hp_trial_mean[0] : host_burst_metric(hp_burst, H, fmt.burst_len),
+                 m1 = on_device ? hp_trial_mean[1] : host_burst_metric(hp_burst + nb_, H, fmt.burst_len);
     det = (m1 < m0) ? 1 : 0;
     th = (det ? m1 : m0) * 4.0;
     const double ph = host_burst_phase(hp_burst + det * nb_, H, fmt);
@@ -898,7 +919,7 @@ bool Context::chroma_fields(ChromaArgs& ca, int P, const DropoutArgs* conceal, u
     const size_t nb = (size_t)H * fmt.burst_len;
     for (int t = 0; t < 2; t++) {
       cudaMemcpyAsync(d_track, hp_trial + t, sizeof(int), cudaMemcpyHostToDevice, cs);
-      chroma_pass(0, 1, false);
+      chroma_pass(0, 1, false, false);
       cudaMemcpyAsync(hp_burst + t * nb, d_burst, nb * sizeof(float), cudaMemcpyDeviceToHost, cs);
     }
     cudaEventRecord(ev_host, cs);
@@ -916,7 +937,7 @@ bool Context::chroma_fields(ChromaArgs& ca, int P, const DropoutArgs* conceal, u
     for (int f = 0; f < P; f++) hp_track[f] = (f & 1) ? (1 - det_track) : det_track;
     cudaMemcpyAsync(d_track, hp_track, P * sizeof(int), cudaMemcpyHostToDevice, cs);
   }
-  chroma_pass(0, P, true);
+  chroma_pass(0, P, true, true);
   cudaEventRecord(ev_host, cs);
   finish(0, P);
   t_host = host_clock();
@@ -942,25 +963,43 @@ bool Context::chroma_fields(ChromaArgs& ca, int P, const DropoutArgs* conceal, u
     h_phase[f] = kPhaseCycle[(cycle_start + f) % 8];
     if (!on_device) computed_track[f] = hp_track[f];
   }
+  // A field's metric depends on its track alone: each is measured once per
+  // track, without its pixels, and the fields whose track then differs from
+  // the plane's are decoded again at the end (a field with no usable burst --
+  // every capture's last, which reaches past its end -- fails on both tracks
+  // and keeps the first pass's pixels).
+  std::vector<double> met[2];
+  std::vector<char> known[2];
+  for (int t = 0; t < 2; t++) {
+    met[t].assign(P, 0.0);
+    known[t].assign(P, 0);
+  }
+  auto note = [&](int f, int track) {
+    met[track][f] = hp_metric[f];
+    known[track][f] = 1;
+  };
+  for (int f = 0; f < P; f++) note(f, computed_track[f]);
+  std::vector<int> plane(P);  // the track the plane ends with
+  std::vector<std::pair<int, int>> again;  // fields to decode again: first, count
   const int fpc = std::max(1, std::min((4096 / H), P));
   for (int f0 = 0; f0 < P; f0 += fpc) {
     const int nf = std::min(fpc, P - f0);
     int retries = 3;
-    bool ok = false;
+    bool ok = false, retried = false;
     while (!ok && retries-- > 0) {
-      bool stale = false;
-      for (int f = f0; f < f0 + nf; f++) stale = stale || computed_track[f] != hp_track[f];
-      if (stale) {
-        cudaMemcpyAsync(d_track + f0, hp_track + f0, nf * sizeof(int), cudaMemcpyHostToDevice, cs);
-        chroma_pass(f0, nf, true);
+      const auto m = chroma_retry_range(f0, nf, H, [&](int f) { return !known[hp_track[f]][f]; });
+      if (m.second > 0) {
+        retried = true;
+        cudaMemcpyAsync(d_track + m.first, hp_track + m.first, m.second * sizeof(int), cudaMemcpyHostToDevice, cs);
+        chroma_pass(m.first, m.second, false, true);
         cudaEventRecord(ev_host, cs);
-        finish(f0, nf);
         if (!wait_host_event("chroma retry")) return false;
-        for (int f = f0; f < f0 + nf; f++) computed_track[f] = hp_track[f];
+        for (int f = m.first; f < m.first + m.second; f++) note(f, hp_track[f]);
       }
+      for (int f = f0; f < f0 + nf; f++) plane[f] = hp_track[f];
       int first_bad = INT_MAX;
       for (int f = 0; f < nf; f++)
-        if (hp_metric[f0 + f] > thr) {
+        if (met[hp_track[f0 + f]][f0 + f] > thr) {
           first_bad = f;
           break;
         }
@@ -971,6 +1010,16 @@ bool Context::chroma_fields(ChromaArgs& ca, int P, const DropoutArgs* conceal, u
         for (int ff = f0 + first_bad; ff < P; ff++) hp_track[ff] = (ff & 1) ? (1 - cur) : cur;
       }
     }
+    if (retried) {
+      const auto m = chroma_redo_range(f0, nf, P, H, [&](int f) { return computed_track[f] != plane[f]; });
+      if (m.second > 0) again.push_back(m);
+    }
+  }
+  for (int f = 0; f < P; f++) hp_track[f] = computed_track[f] = plane[f];
+  for (const auto& m : again) {
+    cudaMemcpyAsync(d_track + m.first, hp_track + m.first, m.second * sizeof(int), cudaMemcpyHostToDevice, cs);
+    chroma_pass(m.first, m.second, true, false);
+    finish(m.first, m.second);
   }
   chroma_valid = true;
   chroma_track = (P & 1) ? (1 - cur) : cur;
@@ -1126,6 +1175,7 @@ bool Context::decode_chunk(const uint8_t* src, bool src_on_device, size_t n_avai
   // and latency bound, and the pre-band-pass (low priority) fills the SMs
   // they leave
   cudaStreamWaitEvent(lstream, ev_k1b, 0);
+  settle_lls(lstream);
   if (debug) cudaMemsetAsync(d_dbg_clk_ll, 0, (size_t)batch * kPhaseSlots * sizeof(long long), lstream);
   auto windows_and_lines = [&](bool again) {
     cudaMemsetAsync(d_counts, 0, 4 * sizeof(int), lstream);
@@ -1337,6 +1387,7 @@ bool Context::decode_chunk(const uint8_t* src, bool src_on_device, size_t n_avai
     tp.fields = P;
     tp.track = d_track;
     tp.pick = d_pick;
+    tp.mean = d_trial_mean;
     launch_track_pick(tp, pstream);
     cudaEventRecord(ev_trial, pstream);
     // the windows and the pick go to the host on the copy stream, so that
@@ -1344,6 +1395,7 @@ bool Context::decode_chunk(const uint8_t* src, bool src_on_device, size_t n_avai
     cudaStreamWaitEvent(xstream, ev_trial, 0);
     cudaMemcpyAsync(hp_burst, d_burst_trial, 2 * nb * sizeof(float), cudaMemcpyDeviceToHost, xstream);
     cudaMemcpyAsync(hp_pick, d_pick, sizeof(int), cudaMemcpyDeviceToHost, xstream);
+    cudaMemcpyAsync(hp_trial_mean, d_trial_mean, 2 * sizeof(double), cudaMemcpyDeviceToHost, xstream);
     cudaEventRecord(ev_trialh, xstream);
   }
   {

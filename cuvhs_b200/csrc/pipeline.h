@@ -7,6 +7,8 @@
 #include <functional>
 #include <memory>
 #include <string>
+#include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "../../include/cuvhs.h"
@@ -23,6 +25,34 @@ constexpr int kGuardPerSlot = 2048;  // near-threshold sync samples one field sl
 
 extern const int kPhaseCycle[8];
 int phase_id_for(int is_first, int quadrant);
+// The chroma line passes transform lines in pairs from a pass's first line, and
+// a line's rounding depends on its partner.  The reference decodes a group of
+// fields [f0, f0 + nf) as one pass on every retry; a pass over part of a group
+// gives the group's values where it starts and ends on the group's pairs.
+// The first of the group's fields for which pick(f) holds, and the count to the
+// last of them, widened to the group's pairs; {f0, 0} if there is none.
+template <class Pick>
+std::pair<int, int> chroma_retry_range(int f0, int nf, int H, Pick pick) {
+  int a = nf, b = 0;
+  for (int i = 0; i < nf; i++)
+    if (pick(f0 + i)) {
+      a = std::min(a, i);
+      b = i + 1;
+    }
+  if (b == 0) return {f0, 0};
+  if ((a * H) & 1) a--;
+  if (((b * H) & 1) && b < nf) b++;
+  return {f0 + a, b - a};
+}
+// The fields of a retried group of a pass over P fields that are to be decoded
+// again: those for which pick(f) holds where the group's pairs are the first
+// pass's, else the whole group.
+template <class Pick>
+std::pair<int, int> chroma_redo_range(int f0, int nf, int P, int H, Pick pick) {
+  const bool same_pairs = ((f0 * H) & 1) == 0 && (f0 + nf == P || ((nf * H) & 1) == 0);
+  if (!same_pairs) return {f0, nf};
+  return chroma_retry_range(f0, nf, H, pick);
+}
 double host_burst_metric(const float* b, int H, int bl);
 double host_burst_phase(const float* b, int H, const Format& fmt);
 
@@ -139,7 +169,9 @@ struct Context {
   int* d_trial = nullptr;        // {0, 1}: the trial tracks
   float* d_burst_trial = nullptr;  // [2][out_h * burst_len]
   int* d_pick = nullptr;
+  double* d_trial_mean = nullptr;
   int* hp_pick = nullptr;
+  double* hp_trial_mean = nullptr;
   uint8_t* d_raw_set[2] = {};
   uint16_t* d_luma_set[2] = {};
   uint16_t* d_chroma_set[2] = {};
@@ -184,6 +216,8 @@ struct Context {
   double* d_vd = nullptr;
   FieldPrep* d_prep = nullptr;
   LineLocState* d_lls = nullptr;
+  bool lls_reset = false;                 // d_lls is to be reset before it is read (settle_lls)
+  LineLocState* hp_lls_fresh = nullptr;   // pinned: a fresh state
   int* d_is_first = nullptr;
   int *d_dbg_vs = nullptr, *d_dbg_vl = nullptr, *d_dbg_vt = nullptr, *d_dbg_vn = nullptr;
   long long *d_dbg_clk_ll = nullptr, *d_dbg_clk_guard = nullptr;  // phase clocks (debug)
@@ -273,6 +307,7 @@ struct Context {
   size_t dev_limit = 0, dev_used = 0;  // device bytes this context may allocate (0: no limit), allocated
   void release();
   void reset_state();
+  void settle_lls(cudaStream_t st);
   bool check_cuda(const char* where);
   bool sync(const char* where);
   bool wait_host_event(const char* where);

@@ -452,18 +452,27 @@ bool Context::decode_round(std::vector<Portion>& ps, const RoundPlan& next_plan)
   if (!wait_host_event("round chroma lines")) return false;
   host_phase(kHostChromaWait, t_host);
   // Per capture, the reference's 15-field groups with up to three retries
-  // each (chroma_decode.cu:782-981), recomputing only fields a flip changed.
-  // The captures advance in lockstep: each runs its host decisions until it
-  // needs a group recomputed, then one launch set over all captures waiting
-  // on a recompute (each on a view of its group's fields) and one wait serve
-  // them together.
+  // each (chroma_decode.cu:782-981).  The captures advance in lockstep: each
+  // runs its host decisions until it needs fields measured on a track they
+  // were not measured on yet, then one launch set over all captures waiting
+  // (each on a view of those fields) and one wait serve them together.  As in
+  // a single decode the measuring leaves the pixels alone; fields whose track
+  // differs from their plane's in the end are decoded again.
   const int fpc_cap = std::max(1, 4096 / H);
   struct Replay {
     int P = 0, fpc = 1, g = 0, it = 0;  // group, iteration within it
-    bool done = true;
-    std::vector<int> computed;
+    int s0 = 0, sn = 0;                 // fields to measure, or to decode again
+    bool done = true, retried = false;
+    std::vector<int> computed, plane;   // the plane's track, and the one it is to have
+    std::vector<std::pair<int, int>> again;  // fields to decode again
+    std::vector<double> met[2];
+    std::vector<char> known[2];
   };
   std::vector<Replay> rp(L);
+  auto note = [&](int j, int f, int track) {
+    rp[j].met[track][f] = hp_metric[ps[live[j]].slot0 + f];
+    rp[j].known[track][f] = 1;
+  };
   for (int j = 0; j < L; j++) {
     const Portion& p = ps[live[j]];
     Replay& r = rp[j];
@@ -471,53 +480,25 @@ bool Context::decode_round(std::vector<Portion>& ps, const RoundPlan& next_plan)
     r.done = r.P == 0;
     r.fpc = std::max(1, std::min(fpc_cap, std::max(r.P, 1)));
     r.computed.assign(hp_track + p.slot0, hp_track + p.slot0 + r.P);
-  }
-  std::vector<int> need;
-  for (;;) {
-    need.clear();
-    for (int j = 0; j < L; j++) {
-      Replay& r = rp[j];
-      const Portion& p = ps[live[j]];
-      int* track = hp_track + p.slot0;
-      const double* metric = hp_metric + p.slot0;
-      while (!r.done) {
-        const int f0 = r.g * r.fpc, nf = std::min(r.fpc, r.P - f0);
-        bool stale = false;
-        for (int f = f0; f < f0 + nf; f++) stale = stale || r.computed[f] != track[f];
-        if (stale) {
-          need.push_back(j);  // recompute, then decide on the new metrics
-          break;
-        }
-        int first_bad = INT_MAX;
-        for (int f = 0; f < nf; f++)
-          if (metric[f0 + f] > thr[j]) {
-            first_bad = f;
-            break;
-          }
-        bool next_group = first_bad == INT_MAX;
-        if (!next_group) {
-          cur[j] = 1 - cur[j];
-          for (int ff = f0 + first_bad; ff < r.P; ff++) track[ff] = (ff & 1) ? (1 - cur[j]) : cur[j];
-          next_group = ++r.it == 3;
-        }
-        if (next_group) {
-          r.g++;
-          r.it = 0;
-          if (r.g * r.fpc >= r.P) r.done = true;
-        }
-      }
+    r.plane = r.computed;
+    for (int t = 0; t < 2; t++) {
+      r.met[t].assign(r.P, 0.0);
+      r.known[t].assign(r.P, 0);
     }
-    if (need.empty()) break;
-    static thread_local ArgsMany<ChromaArgs> cv;
-    static thread_local ArgsMany<DropoutArgs> ov;
+    for (int f = 0; f < r.P; f++) note(j, f, r.computed[f]);
+  }
+  static thread_local ArgsMany<ChromaArgs> cv;
+  static thread_local ArgsMany<DropoutArgs> ov;
+  std::vector<int> need;
+  // one launch set over fields [s0, s0 + sn) of every capture in `need`
+  auto group_pass = [&](bool write) {
     int max_nf = 0;
     for (size_t q = 0; q < need.size(); q++) {
       const int j = need[q];
-      const Replay& r = rp[j];
-      const int f0 = r.g * r.fpc, nf = std::min(r.fpc, r.P - f0);
+      const int f0 = rp[j].s0, nf = rp[j].sn;
       max_nf = std::max(max_nf, nf);
-      const int s0 = ps[live[j]].slot0;
-      cudaMemcpyAsync(d_track + s0 + f0, hp_track + s0 + f0, nf * sizeof(int), cudaMemcpyHostToDevice, stream);
+      const int slot = ps[live[j]].slot0;
+      cudaMemcpyAsync(d_track + slot + f0, hp_track + slot + f0, nf * sizeof(int), cudaMemcpyHostToDevice, stream);
       // the capture's fields [f0, f0 + nf) as a capture of nf fields
       ChromaArgs c = cm.a[j];
       c.ll += (size_t)f0 * LPF;
@@ -542,22 +523,78 @@ bool Context::decode_round(std::vector<Portion>& ps, const RoundPlan& next_plan)
     const int nq = (int)need.size();
     cudaEvent_t ev_;
     begin_stage(kStageChromaLines, ev_);
-    launch_chroma_lines_many(cv, nq, -1, max_nf, true, stream);
+    launch_chroma_lines_many(cv, nq, -1, max_nf, write, stream);
     end_stage(kStageChromaLines, ev_);
-    begin_stage(kStageBurstMetric, ev_);
-    launch_burst_metric_many(cv, nq, max_nf, stream);
-    end_stage(kStageBurstMetric, ev_);
-    begin_stage(kStageDropouts, ev_);
-    launch_dropout_conceal_chroma_many(ov, nq, max_nf, stream);
-    end_stage(kStageDropouts, ev_);
+    if (write) {
+      begin_stage(kStageDropouts, ev_);
+      launch_dropout_conceal_chroma_many(ov, nq, max_nf, stream);
+      end_stage(kStageDropouts, ev_);
+    } else {
+      begin_stage(kStageBurstMetric, ev_);
+      launch_burst_metric_many(cv, nq, max_nf, stream);
+      end_stage(kStageBurstMetric, ev_);
+    }
+  };
+  for (;;) {
+    need.clear();
+    for (int j = 0; j < L; j++) {
+      Replay& r = rp[j];
+      const Portion& p = ps[live[j]];
+      int* track = hp_track + p.slot0;
+      while (!r.done) {
+        const int f0 = r.g * r.fpc, nf = std::min(r.fpc, r.P - f0);
+        const auto m = chroma_retry_range(f0, nf, H, [&](int f) { return !r.known[track[f]][f]; });
+        if (m.second > 0) {
+          r.s0 = m.first;
+          r.sn = m.second;
+          r.retried = true;
+          need.push_back(j);  // measure, then decide
+          break;
+        }
+        std::copy(track + f0, track + f0 + nf, r.plane.begin() + f0);
+        int first_bad = INT_MAX;
+        for (int f = 0; f < nf; f++)
+          if (r.met[track[f0 + f]][f0 + f] > thr[j]) {
+            first_bad = f;
+            break;
+          }
+        bool next_group = first_bad == INT_MAX;
+        if (!next_group) {
+          cur[j] = 1 - cur[j];
+          for (int ff = f0 + first_bad; ff < r.P; ff++) track[ff] = (ff & 1) ? (1 - cur[j]) : cur[j];
+          next_group = ++r.it == 3;
+        }
+        if (next_group) {
+          if (r.retried) {
+            const auto redo = chroma_redo_range(f0, nf, r.P, H, [&](int f) { return r.computed[f] != r.plane[f]; });
+            if (redo.second > 0) r.again.push_back(redo);
+          }
+          r.retried = false;
+          r.g++;
+          r.it = 0;
+          if (r.g * r.fpc >= r.P) r.done = true;
+        }
+      }
+    }
+    if (need.empty()) break;
+    group_pass(false);
     cudaEventRecord(ev_host, stream);
     if (!wait_host_event("round chroma retry")) return false;
-    for (int j : need) {
-      Replay& r = rp[j];
-      const int f0 = r.g * r.fpc, nf = std::min(r.fpc, r.P - f0);
-      const int* track = hp_track + ps[live[j]].slot0;
-      for (int f = f0; f < f0 + nf; f++) r.computed[f] = track[f];
-    }
+    for (int j : need)
+      for (int f = rp[j].s0; f < rp[j].s0 + rp[j].sn; f++) note(j, f, hp_track[ps[live[j]].slot0 + f]);
+  }
+  // fields to decode again, a run of each capture per launch set
+  for (int j = 0; j < L; j++) std::copy(rp[j].plane.begin(), rp[j].plane.end(), hp_track + ps[live[j]].slot0);
+  for (size_t k = 0;; k++) {
+    need.clear();
+    for (int j = 0; j < L; j++)
+      if (k < rp[j].again.size()) {
+        rp[j].s0 = rp[j].again[k].first;
+        rp[j].sn = rp[j].again[k].second;
+        need.push_back(j);
+      }
+    if (need.empty()) break;
+    group_pass(true);
   }
   // chroma planes out
   cudaEventRecord(ev_chroma, stream);

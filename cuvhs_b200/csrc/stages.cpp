@@ -163,6 +163,7 @@ cuvhs_status cuvhs_stage_line_locations(cuvhs_ctx* ctx, uint64_t raw_offset, con
   cudaMemcpyAsync(c.d_pl, lengths, np * sizeof(int), cudaMemcpyHostToDevice, c.stream);
   cudaMemcpyAsync(c.d_pn, pn.data(), n_fields * sizeof(int), cudaMemcpyHostToDevice, c.stream);
   cuvhs::LineLocArgs la = c.lineloc_args(n_fields, n_fields, (long long)raw_offset);
+  c.settle_lls(c.stream);
   cuvhs::launch_line_locations(la, c.stream);
   std::vector<int32_t> first(n_fields);
   cudaMemcpyAsync(linelocs, c.d_ll, (size_t)n_fields * LPF * sizeof(double), cudaMemcpyDeviceToHost, c.stream);
