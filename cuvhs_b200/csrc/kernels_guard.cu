@@ -23,8 +23,8 @@
 // sync sum reads split into a few runs -- consecutive chunk positions of one
 // owning tile, or one clamped position repeated -- and each run's analytic
 // signal is one FP64 overlap-save convolution: its raw window (tile wrap and
-// chunk clamp applied per sample) goes through a 4096-point FP64 FFT in shared
-// memory, is multiplied by the FFT of the truncated taps and transformed back,
+// chunk clamp applied per sample) goes through a 4096-point FP64 FFT (registers and shared
+// memory), is multiplied by the FFT of the truncated taps and transformed back,
 // giving every z of up to 4095 - 2*ha consecutive positions at once.  The
 // phase differences fill a demod array indexed like the sync taps, and the
 // sync sum is taken in a fixed order, so the result is deterministic.
@@ -39,13 +39,15 @@
 namespace cuvhs {
 namespace {
 
-constexpr int kGT = 512;                  // threads per CTA (two CTAs per SM)
+constexpr int kGT = 256;                  // threads per CTA: 16 points each (two CTAs per SM)
 constexpr int kN = Design::kGuardN;       // FFT length
-constexpr int kBfly = kN / 4 / kGT;       // radix-4 butterflies per thread per pass
+constexpr int kRow = 16 * 17 + 1;         // padded slots of 256 points: one after every 16 and every 256
+constexpr int kSlots = 16 * kRow;         // the padded transform
 constexpr int kTwQ = kN / 4;              // twiddles held in shared memory: exp(-2 pi i k / kN), k < kN / 4
+constexpr int kTwPad = kTwQ + kTwQ / 8;   // one slot after every 8
 constexpr double kPi64 = 3.14159265358979323846;
 constexpr double kTau64 = 2.0 * kPi64;
-static_assert(kN == 4096 && kBfly >= 1 && kN / 4 % kGT == 0, "the FFT passes assume 4096 points");
+static_assert(kN == 4096 && kGT == 256, "three passes of 16 points on 256 threads");
 
 __device__ __forceinline__ long long wrap_pos(long long q, long long tile) {
   return q < 0 ? q + tile : (q >= tile ? q - tile : q);
@@ -55,57 +57,119 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// exp(-2 pi i j / kN) for j < 3 kN / 4 from the quarter table: the quadrant
-// q = j / (kN / 4) multiplies by (-i)^q.
-__device__ __forceinline__ double2 twiddle(const double2* tq, int j) {
-  const double2 w = tq[j & (kTwQ - 1)];
-  switch (j / kTwQ) {
-    case 0: return w;
-    case 1: return make_double2(w.y, -w.x);
-    default: return make_double2(-w.x, -w.y);
-  }
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+// a * (-i), conjugated for the inverse
+template <bool kInverse>
+__device__ __forceinline__ double2 turn(double2 a) {
+  return kInverse ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
 }
 
-// In-place radix-4 Stockham FFT of kN points in shared memory (every thread
-// holds its butterflies' inputs in registers across a barrier, so one buffer
-// serves as source and destination).  tq: the quarter twiddle table; the
-// inverse conjugates the twiddles and is unnormalised.
+// exp(-2 pi i j / kN) for j < kN from the quarter table: the quadrant
+// q = j / (kN / 4) multiplies by (-i)^q.  The inverse conjugates.
 template <bool kInverse>
-__device__ void fft_n(double2* buf, const double2* tq) {
-  const int t = threadIdx.x;
-  for (int ns = 1; ns < kN; ns *= 4) {
-    double2 v[kBfly][4];
+__device__ __forceinline__ double2 twiddle(const double2* tq, int j) {
+  const int m = j & (kTwQ - 1), q = j / kTwQ;
+  const double2 w = tq[m + (m >> 3)];
+  double2 r = (q & 1) ? make_double2(w.y, -w.x) : w;
+  if (q & 2) r = make_double2(-r.x, -r.y);
+  return kInverse ? make_double2(r.x, -r.y) : r;
+}
+
+// Four-point DFT of v[0], v[S], v[2S], v[3S] in place.
+template <bool kInverse, int S>
+__device__ __forceinline__ void dft4(double2* v) {
+  const double2 s02 = cadd(v[0], v[2 * S]), d02 = csub(v[0], v[2 * S]);
+  const double2 s13 = cadd(v[S], v[3 * S]), m = turn<kInverse>(csub(v[S], v[3 * S]));
+  v[0] = cadd(s02, s13);
+  v[S] = cadd(d02, m);
+  v[2 * S] = csub(s02, s13);
+  v[3 * S] = csub(d02, m);
+}
+
+// Sixteen-point DFT; output k is left in v[4 * (k & 3) + (k >> 2)] (slot16).
+__device__ __forceinline__ constexpr int slot16(int k) { return 4 * (k & 3) + (k >> 2); }
+
+template <bool kInverse>
+__device__ __forceinline__ void dft16(double2 (&v)[16]) {
+  constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173;  // cos, sin of pi / 8
+  constexpr double h = 0.70710678118654752440;
+  constexpr double sg = kInverse ? 1.0 : -1.0;
 #pragma unroll
-    for (int b = 0; b < kBfly; b++) {
-      const int j = t + b * kGT;
+  for (int c = 0; c < 4; c++) dft4<kInverse, 4>(v + c);  // v[4 r + c] -> r
+  auto w8 = [](double2 a) {  // times exp(-+ i pi / 4)
+    const double2 t = turn<kInverse>(a);
+    return make_double2((a.x + t.x) * h, (a.y + t.y) * h);
+  };
+  v[5] = cmul(v[5], make_double2(c1, sg * s1));
+  v[6] = w8(v[6]);
+  v[7] = cmul(v[7], make_double2(s1, sg * c1));
+  v[9] = w8(v[9]);
+  v[10] = turn<kInverse>(v[10]);
+  v[11] = turn<kInverse>(w8(v[11]));
+  v[13] = cmul(v[13], make_double2(s1, sg * c1));
+  v[14] = turn<kInverse>(w8(v[14]));
+  v[15] = cmul(v[15], make_double2(-c1, -sg * s1));
 #pragma unroll
-      for (int r = 0; r < 4; r++) v[b][r] = buf[j + r * (kN / 4)];
-    }
-    __syncthreads();
-    const int stride = kN / (4 * ns);
+  for (int r = 0; r < 4; r++) dft4<kInverse, 1>(v + 4 * r);
+}
+
+// The block's convolution: v[i] holds the real input at position t + 256 i;
+// on return buf[t + 256 i] (padded: slot_of) holds the analytic signal there.
+//
+// FP64 multiply-adds and shared memory traffic bound a transform: three passes
+// of 16 points in registers touch shared memory twice per transform (six
+// radix-4 passes through it, on 512 threads, took the whole kernel from 36.2
+// us to 27.9 for a 3-tile chunk, from 60.1 to 40.1 for 24 tiles at 35.8 MHz).
+// A pass reads and writes its own slots, so one barrier per pass suffices; the
+// spectrum leaves the third pass in the order the inverse's first pass takes,
+// so the filter is applied in registers.  The padding keeps a warp's slots of
+// every pass and of the first pass's twiddles (strides 0..15) on distinct banks
+// (quarter warps of 16-byte accesses).
+__device__ __forceinline__ int slot_of(int n) { return n + (n >> 4) + (n >> 8); }
+
+__device__ __forceinline__ void convolve(double2 (&v)[16], double2* buf, const double2* tq, const double2* tw2,
+                                         const double2* __restrict__ gfft) {
+  const int t = threadIdx.x, lo = t & 15, hi = t >> 4;
+  double2* const col = buf + t + hi;              // pass 1: position t + 256 i, i along kRow
+  double2* const mid = buf + hi * kRow + lo;      // pass 2: row hi, position lo + 16 i, i along 17
+  double2* const row = buf + lo * kRow + hi * 17; // pass 3: row lo, positions 16 hi + i
+  dft16<false>(v);
 #pragma unroll
-    for (int b = 0; b < kBfly; b++) {
-      const int j = t + b * kGT;
-      const int k = j & (ns - 1);
+  for (int k = 0; k < 16; k++) col[k * kRow] = k ? cmul(v[slot16(k)], twiddle<false>(tq, k * t)) : v[0];
+  __syncthreads();
 #pragma unroll
-      for (int r = 1; r < 4; r++) {
-        double2 w = twiddle(tq, r * k * stride);
-        if (kInverse) w.y = -w.y;
-        v[b][r] = cmul(v[b][r], w);
-      }
-      const double2 a0 = v[b][0], a1 = v[b][1], a2 = v[b][2], a3 = v[b][3];
-      const double2 s02 = make_double2(a0.x + a2.x, a0.y + a2.y), d02 = make_double2(a0.x - a2.x, a0.y - a2.y);
-      const double2 s13 = make_double2(a1.x + a3.x, a1.y + a3.y), d13 = make_double2(a1.x - a3.x, a1.y - a3.y);
-      // forward: X1 = d02 - i d13, X3 = d02 + i d13; the inverse swaps them
-      const double2 m = kInverse ? make_double2(-d13.y, d13.x) : make_double2(d13.y, -d13.x);  // -/+ i d13
-      const int base = (j / ns) * ns * 4 + k;
-      buf[base] = make_double2(s02.x + s13.x, s02.y + s13.y);
-      buf[base + ns] = make_double2(d02.x + m.x, d02.y + m.y);
-      buf[base + 2 * ns] = make_double2(s02.x - s13.x, s02.y - s13.y);
-      buf[base + 3 * ns] = make_double2(d02.x - m.x, d02.y - m.y);
-    }
-    __syncthreads();
+  for (int i = 0; i < 16; i++) v[i] = mid[i * 17];
+  dft16<false>(v);
+#pragma unroll
+  for (int k = 0; k < 16; k++) mid[k * 17] = k ? cmul(v[slot16(k)], tw2[k * 16 + lo]) : v[0];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 16; i++) v[i] = row[i];
+  dft16<false>(v);
+  double2 g[16];
+#pragma unroll
+  for (int k = 0; k < 16; k++) g[k] = cmul(v[slot16(k)], __ldg(&gfft[t + 256 * k]));  // frequency lo + 16 hi + 256 k
+  dft16<true>(g);
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    double2 w = tw2[hi * 16 + i];
+    w.y = -w.y;
+    row[i] = cmul(g[slot16(i)], w);
   }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 16; i++) v[i] = mid[i * 17];
+  dft16<true>(v);
+#pragma unroll
+  for (int i = 0; i < 16; i++) mid[i * 17] = cmul(v[slot16(i)], twiddle<true>(tq, hi * (lo + 16 * i)));
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 16; i++) v[i] = col[i * kRow];
+  dft16<true>(v);
+#pragma unroll
+  for (int i = 0; i < 16; i++) col[i * kRow] = v[slot16(i)];
+  __syncthreads();
 }
 
 // A run of the sample's demod positions: taps kk0..kk1 read chunk position
@@ -127,9 +191,10 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
   const GuardArgs& g = src.get();
   chain_wait();
   extern __shared__ double2 gsm[];
-  double2* buf = gsm;                                        // [kN]
-  double2* tq = gsm + kN;                                    // [kTwQ]
-  double* dem = reinterpret_cast<double*>(gsm + kN + kTwQ);  // [2 * hb + 1], indexed like the sync taps
+  double2* buf = gsm;             // [kSlots]
+  double2* tq = buf + kSlots;     // [kTwPad] exp(-2 pi i k / 4096), padded
+  double2* tw2 = tq + kTwPad;     // [16][16] exp(-2 pi i k j / 256)
+  double* dem = reinterpret_cast<double*>(tw2 + 256);  // [2 * hb + 1], indexed like the sync taps
   __shared__ Run runs[kMaxRuns];
   __shared__ int nruns, skip;
   __shared__ double red[kGT / 32];
@@ -140,7 +205,8 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
   const int W = 2 * g.hb + 1;
   const int V = kN - 1 - 2 * g.ha;  // demod positions one FFT block yields
   if ((int)blockIdx.x >= n_listed) return;  // whole CTA
-  for (int k = t; k < kTwQ; k += kGT) tq[k] = __ldg(&g.tw[k]);
+  for (int k = t; k < kTwQ; k += kGT) tq[k + (k >> 3)] = __ldg(&g.tw[k]);
+  tw2[t] = __ldg(&g.tw[16 * (t & 15) * (t >> 4)]);
   __syncthreads();
   for (int y = blockIdx.x; y < n_listed; y += gridDim.x) {
     const long long s = g.list[y];
@@ -214,33 +280,31 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
         const int nz = (int)(ce - cb) + 2;             // z at tile positions J2(cb) - 1 .. J2(ce)
         const long long v0 = (kOverlap + cb - owner * g.spp) - 1 - g.ha;  // tile position of buf[0]
         const int L = nz + 2 * g.ha;
-        for (int u = t; u < kN; u += kGT) {
+        double2 v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          const int u = t + i * kGT;
           double x = 0.0;
           if (u < L) {
             const long long p = min(max(tile0 + wrap_pos(v0 + u, g.tile), 0LL), last);
             x = p < g.n_read ? (double)raw_convert<FMT>(g.raw, (int)p) - dc : 0.0;
           }
-          buf[u] = make_double2(x, 0.0);
+          v[i] = make_double2(x, 0.0);
         }
-        __syncthreads();
         const bool first_block = r == 0 && cb == c_lo;
         if (first_block) phase_clock(g, y, 1);
-        fft_n<false>(buf, tq);
+        convolve(v, buf, tq, tw2, g.gfft);
         if (first_block) phase_clock(g, y, 2);
-#pragma unroll
-        for (int k = t; k < kN; k += kGT) buf[k] = cmul(buf[k], __ldg(&g.gfft[k]));
-        __syncthreads();
-        fft_n<true>(buf, tq);
-        if (first_block) phase_clock(g, y, 3);
         // phases of the block's z, in place
         for (int i = t; i < nz; i += kGT) {
-          const double2 z = buf[g.ha + i];
-          buf[g.ha + i].x = atan2(z.y, z.x);
+          double2& z = buf[slot_of(g.ha + i)];
+          z.x = atan2(z.y, z.x);
         }
         __syncthreads();
+        if (first_block) phase_clock(g, y, 3);
         // k_unwrap_to_hz (fm_demod.cu:222-244) for chunk positions cb .. ce
         for (int i = t; i + 1 < nz; i += kGT) {
-          double d = buf[g.ha + i + 1].x - buf[g.ha + i].x;
+          double d = buf[slot_of(g.ha + i + 1)].x - buf[slot_of(g.ha + i)].x;
           if (d > kPi64) d -= kTau64;
           if (d < -kPi64) d += kTau64;
           const double hz = d * g.scale;
@@ -284,7 +348,7 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
 }  // namespace
 
 size_t guard_smem_bytes(int hb) {
-  return (size_t)(kN + kTwQ) * sizeof(double2) + (size_t)(2 * hb + 1) * sizeof(double);
+  return (size_t)(kSlots + kTwPad + 256) * sizeof(double2) + (size_t)(2 * hb + 1) * sizeof(double);
 }
 
 bool guard_supported(int ha, int hb) {
