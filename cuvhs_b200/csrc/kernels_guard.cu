@@ -49,7 +49,7 @@ constexpr double kPi64 = 3.14159265358979323846;
 constexpr double kTau64 = 2.0 * kPi64;
 static_assert(kN == 4096 && kGT == 256, "three passes of 16 points on 256 threads");
 
-__device__ __forceinline__ long long wrap_pos(long long q, long long tile) {
+__device__ __forceinline__ int wrap_pos(int q, int tile) {
   return q < 0 ? q + tile : (q >= tile ? q - tile : q);
 }
 
@@ -120,7 +120,7 @@ __device__ __forceinline__ void dft16(double2 (&v)[16]) {
 // FP64 multiply-adds and shared memory traffic bound a transform: three passes
 // of 16 points in registers touch shared memory twice per transform (six
 // radix-4 passes through it, on 512 threads, took the whole kernel from 36.2
-// us to 27.9 for a 3-tile chunk, from 60.1 to 40.1 for 24 tiles at 35.8 MHz).
+// us to 26.4 for a 3-tile chunk, from 60.1 to 37.6 for 24 tiles at 35.8 MHz).
 // A pass reads and writes its own slots, so one barrier per pass suffices; the
 // spectrum leaves the third pass in the order the inverse's first pass takes,
 // so the filter is applied in registers.  The padding keeps a warp's slots of
@@ -189,7 +189,6 @@ __device__ __forceinline__ void phase_clock(const GuardArgs& g, int y, int k) {
 template <int FMT, class Src>
 __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ Src src) {
   const GuardArgs& g = src.get();
-  chain_wait();
   extern __shared__ double2 gsm[];
   double2* buf = gsm;             // [kSlots]
   double2* tq = buf + kSlots;     // [kTwPad] exp(-2 pi i k / 4096), padded
@@ -198,19 +197,20 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
   __shared__ Run runs[kMaxRuns];
   __shared__ int nruns, skip;
   __shared__ double red[kGT / 32];
-  const int n_listed = min(*g.count, g.cap);
   const int t = threadIdx.x;
+  // the tables are the context's: staged before the wait for the launch ahead
+  for (int k = t; k < kTwQ; k += kGT) tq[k + (k >> 3)] = __ldg(&g.tw[k]);
+  tw2[t] = __ldg(&g.tw[16 * (t & 15) * (t >> 4)]);
+  chain_wait();
+  const int n_listed = min(*g.count, g.cap);
   const double dc = g.dc ? (double)*g.dc : 0.0;
   const long long last = g.total - 1;
   const int W = 2 * g.hb + 1;
   const int V = kN - 1 - 2 * g.ha;  // demod positions one FFT block yields
   if ((int)blockIdx.x >= n_listed) return;  // whole CTA
-  for (int k = t; k < kTwQ; k += kGT) tq[k + (k >> 3)] = __ldg(&g.tw[k]);
-  tw2[t] = __ldg(&g.tw[16 * (t & 15) * (t >> 4)]);
-  __syncthreads();
   for (int y = blockIdx.x; y < n_listed; y += gridDim.x) {
     const long long s = g.list[y];
-    const long long f = s / g.spp;
+    const long long f = (unsigned)s / (unsigned)g.spp;  // chunk positions fit 32 bits
     const long long J = kOverlap + (s - f * g.spp);
     phase_clock(g, y, 0);
     if (t == 0) {
@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
             kend = kk1;
             runs[n++] = {kk, kend, 0, 0};
           } else {
-            const long long stop = (c / g.spp) * g.spp;  // the owning tile's first position
+            // the owning tile's first position
+            const long long stop = (long long)((unsigned)c / (unsigned)g.spp) * g.spp;
             kend = (int)min((long long)kk1, kk + (c - stop));
             runs[n++] = {kk, kend, -1, c};
           }
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
       int sk = 0;
       if (g.n_read < g.total) {
         for (int r = 0; r < n; r++) {
-          const long long owner = runs[r].c0 / g.spp;
+          const long long owner = (unsigned)runs[r].c0 / (unsigned)g.spp;
           const long long tile0 = owner * g.spp - kOverlap;
           const long long vmax = (kOverlap + runs[r].c0 - owner * g.spp) + g.ha;  // highest tile position read
           const long long pmax = min(tile0 + min(vmax, (long long)g.tile - 1), last);
@@ -273,21 +274,25 @@ __global__ void __launch_bounds__(kGT, 2) guard_kernel(const __grid_constant__ S
     for (int r = 0; r < nruns; r++) {
       const Run run = runs[r];
       const long long c_hi = run.c0, c_lo = run.c0 + (long long)run.step * (run.kk1 - run.kk0);
-      const long long owner = c_lo / g.spp;
+      const long long owner = (unsigned)c_lo / (unsigned)g.spp;
       const long long tile0 = owner * g.spp - kOverlap;  // chunk position of the owner's tile position 0
       for (long long cb = c_lo; cb <= c_hi; cb += V) {
         const long long ce = min(cb + V - 1, c_hi);
         const int nz = (int)(ce - cb) + 2;             // z at tile positions J2(cb) - 1 .. J2(ce)
         const long long v0 = (kOverlap + cb - owner * g.spp) - 1 - g.ha;  // tile position of buf[0]
         const int L = nz + 2 * g.ha;
+        // tile positions clamped to the chunk, and those read, as offsets from the tile's start
+        const int q_lo = (int)max(-tile0, 0LL), q_hi = (int)min(last - tile0, (long long)g.tile - 1);
+        const int q_read = (int)min((long long)g.n_read - tile0, (long long)g.tile);
+        const uint8_t* const raw0 = g.raw + tile0 * (FMT == kInU8 ? 1 : 2);
         double2 v[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) {
           const int u = t + i * kGT;
           double x = 0.0;
           if (u < L) {
-            const long long p = min(max(tile0 + wrap_pos(v0 + u, g.tile), 0LL), last);
-            x = p < g.n_read ? (double)raw_convert<FMT>(g.raw, (int)p) - dc : 0.0;
+            const int q = min(max(wrap_pos((int)v0 + u, (int)g.tile), q_lo), q_hi);
+            x = q < q_read ? (double)raw_convert<FMT>(raw0, q) - dc : 0.0;
           }
           v[i] = make_double2(x, 0.0);
         }
