@@ -99,6 +99,8 @@ constexpr int kMaxFieldLines = 320;  // line starts held in shared memory: 264 N
 struct MapScratch {
   double ll[kMaxFieldLines];  // the field's line starts from the first active line
   int rf_s[kMaxRfDropouts], rf_e[kMaxRfDropouts];
+  int sl[kMaxRfDropouts], el[kMaxRfDropouts];  // lines each span touches
+  int base[kMaxRfDropouts];                    // lines of the spans before it
   int wsh[32];
 };
 
@@ -125,11 +127,14 @@ __device__ __forceinline__ bool span_entry(const double* ll, int l, int sl, int 
 // "no dropout", so events 2i and 2i + 1 are the start and end of run i (the
 // last may lack its end: the range's end); a run joins the one before it when
 // its start lies within 30 samples of that one's end, so the spans are the
-// runs numbered by a prefix sum, and a span's entries go behind those of the
-// spans before it by another.  Latency bound (a few hundred events at most,
-// a few KB): one thread walking the events with each line search in global
-// memory took 0.5 ms for a field that reaches past the capture's end; the
-// searches now read shared memory, a thread per span.
+// runs numbered by a prefix sum; the lines the spans touch, in the spans'
+// order, are numbered by a second one and taken a thread each, their entries
+// placed by a third.  Latency bound (a few hundred events at most, a few KB):
+// one thread walking the events with each line search in global memory took
+// 0.5 ms for a field that reaches past the capture's end, whose one span
+// touches every line; with a thread per span walking its lines, and the
+// concealment below testing every entry in every column, the dropout stage of
+// 16 PAL fields took 154 us, now 79.
 template <int THREADS>
 __device__ void map_events(const DropoutArgs& a, int f, const int* events, int ne, int s0, int s1, MapScratch& m) {
   static_assert(THREADS >= kMaxRfDropouts, "a thread per span");
@@ -152,31 +157,51 @@ __device__ void map_events(const DropoutArgs& a, int f, const int* events, int n
   }
   nrf = min(nrf, kMaxRfDropouts);
   __syncthreads();
-  int sl = 0, el = -1, cnt = 0, sx, ex;
-  double sa = 0.0, ea = 0.0;
+  int sl = 0, el = -1;
   if (tid < nrf && m.rf_e[tid] - m.rf_s[tid] >= 10) {
-    sa = (double)m.rf_s[tid];
-    ea = (double)m.rf_e[tid];
-    sl = find_line(m.ll, H, sa);
+    sl = find_line(m.ll, H, (double)m.rf_s[tid]);
     if (sl >= 0) {
-      el = find_line(m.ll, H, ea - 1.0);
+      el = find_line(m.ll, H, (double)m.rf_e[tid] - 1.0);
       if (el < 0) el = H - 1;
-      for (int l = sl; l <= el; l++) cnt += span_entry(m.ll, l, sl, el, sa, ea, W, sx, ex) ? 1 : 0;
     }
   }
-  int n;
-  int k = block_excl_sum<THREADS>(cnt, m.wsh, &n);
+  const int cnt = sl >= 0 ? max(el - sl + 1, 0) : 0;
+  int lines;
+  const int base = block_excl_sum<THREADS>(cnt, m.wsh, &lines);
+  if (tid < nrf) {
+    m.sl[tid] = sl;
+    m.el[tid] = el;
+    m.base[tid] = base;
+  }
+  __syncthreads();
   int* ol = a.do_lines + (size_t)f * kMaxDropouts;
   int* os = a.do_starts + (size_t)f * kMaxDropouts;
   int* oe = a.do_ends + (size_t)f * kMaxDropouts;
-  if (cnt > 0)
-    for (int l = sl; l <= el && k < kMaxDropouts; l++)
-      if (span_entry(m.ll, l, sl, el, sa, ea, W, sx, ex)) {
-        ol[k] = l;
-        os[k] = sx;
-        oe[k] = ex;
-        k++;
+  int n = 0;
+  for (int j0 = 0; j0 < lines && n < kMaxDropouts; j0 += THREADS) {
+    const int j = j0 + tid;
+    bool ok = false;
+    int l = 0, sx = 0, ex = 0;
+    if (j < lines) {
+      // the last span whose lines start at or before j (one without lines shares the next one's base)
+      int lo = 0, hi = nrf - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (m.base[mid] <= j) lo = mid;
+        else hi = mid - 1;
       }
+      l = m.sl[lo] + j - m.base[lo];
+      ok = span_entry(m.ll, l, m.sl[lo], m.el[lo], (double)m.rf_s[lo], (double)m.rf_e[lo], W, sx, ex);
+    }
+    int total;
+    const int k = n + block_excl_sum<THREADS>(ok ? 1 : 0, m.wsh, &total);
+    if (ok && k < kMaxDropouts) {
+      ol[k] = l;
+      os[k] = sx;
+      oe[k] = ex;
+    }
+    n += total;
+  }
   if (tid == 0) a.do_count[f] = min(n, kMaxDropouts);
 }
 
@@ -189,9 +214,13 @@ __device__ void map_events(const DropoutArgs& a, int f, const int* events, int n
 // step; the smallest such sx_e wrote last), what e's source row held at e's
 // step.  Each pixel's origin therefore follows from the entries alone, and
 // columns never mix: a thread takes a column through all groups in order,
-// the group's loads all in flight before its stores.  Latency bound; a warp
-// stepping through the columns took 0.7 us a step, 1.4 ms for a field with
-// 512 entries.
+// the group's loads all in flight before its stores.  A warp takes 32 columns:
+// its lanes first look at the group's entries against those columns, so that
+// entries elsewhere cost a test each, and one that covers them all with no
+// other entry on its rows (a dropout of whole lines) a load and a store.
+// Issue bound on the one SM of a field with many entries, latency bound
+// otherwise; a warp stepping through the columns took 0.7 us a step, 1.4 ms
+// for a field with 512 entries.
 struct ConcealEntry {
   short line, src, sx, ex;
   unsigned before;  // entries of the group on row src with a larger sx
@@ -229,24 +258,47 @@ __device__ void conceal_entries(const DropoutArgs& a, int f, int n, ConcealEntry
 
 __device__ __forceinline__ bool covers(const ConcealEntry& e, int c) { return c >= e.sx && c < e.ex; }
 
-// Column c of one plane through every group of entries.
-__device__ void conceal_column(const ConcealEntry* ent, int n, uint16_t* plane, int W, int c) {
+// Columns [c0, c0 + 32) of one plane through every group of entries (whole warp).
+__device__ void conceal_columns(const ConcealEntry* ent, int n, uint16_t* plane, int W, int c0) {
+  const int lane = threadIdx.x & 31;
+  const int c = c0 + lane;
+  const int c_end = min(c0 + 32, W);
   for (int g = 0; g < n; g += 32) {
-    const int m = min(32, n - g);
+    int src = 0, dst = 0;
+    unsigned links = 0;
+    bool touch = false, whole = false;
+    if (g + lane < n) {
+      const ConcealEntry e = ent[g + lane];
+      touch = e.sx < c_end && e.ex > c0;
+      whole = e.sx <= c0 && e.ex >= c_end;
+      links = e.before | e.after;
+      src = e.src * W;
+      dst = e.line * W;
+    }
+    const unsigned any = __ballot_sync(0xffffffffu, touch);
+    if (!any) continue;
+    const unsigned plain = __ballot_sync(0xffffffffu, whole && (links & any) == 0);
     uint16_t v[32];
     unsigned act = 0;
 #pragma unroll
     for (int d = 0; d < 32; d++) {
       v[d] = 0;
-      if (d >= m) continue;
+      if (!(any >> d & 1u)) continue;
+      const int row_d = __shfl_sync(0xffffffffu, src, d);
+      if (c >= W) continue;
+      if (plain >> d & 1u) {
+        act |= 1u << d;
+        v[d] = plane[row_d + c];
+        continue;
+      }
       const ConcealEntry e = ent[g + d];
       if (!covers(e, c)) continue;
       bool last = true;  // no later write of the group to this pixel
-      for (unsigned w = e.after; w; w &= w - 1) last = last && !covers(ent[g + __ffs(w) - 1], c);
+      for (unsigned w = e.after & any; w; w &= w - 1) last = last && !covers(ent[g + __ffs(w) - 1], c);
       if (!last) continue;
       act |= 1u << d;
       int row = e.src;
-      for (unsigned w = e.before; w;) {
+      for (unsigned w = e.before & any; w;) {
         int best = -1, bsx = 1 << 30;
         for (; w; w &= w - 1) {
           const int k = __ffs(w) - 1;
@@ -257,14 +309,17 @@ __device__ void conceal_column(const ConcealEntry* ent, int n, uint16_t* plane, 
         }
         if (best >= 0) {
           row = ent[g + best].src;
-          w = ent[g + best].before;
+          w = ent[g + best].before & any;
         }
       }
       v[d] = plane[row * W + c];
     }
 #pragma unroll
-    for (int d = 0; d < 32; d++)
-      if (act >> d & 1u) plane[ent[g + d].line * W + c] = v[d];
+    for (int d = 0; d < 32; d++) {
+      if (!(any >> d & 1u)) continue;
+      const int row_d = __shfl_sync(0xffffffffu, dst, d);
+      if (act >> d & 1u) plane[row_d + c] = v[d];
+    }
   }
 }
 
@@ -347,9 +402,9 @@ __global__ void __launch_bounds__(kThreadsD) dropout_kernel(DropoutArgs a) {
   if (n <= 0) return;  // whole CTA
   conceal_entries<kThreadsD>(a, f, n, ent);
   const size_t F = (size_t)a.out_h * a.out_w;
-  for (int c = tid; c < a.out_w; c += kThreadsD) {
-    conceal_column(ent, n, a.luma + f * F, a.out_w, c);
-    conceal_column(ent, n, a.chroma + f * F, a.out_w, c);
+  for (int c0 = tid & ~31; c0 < a.out_w; c0 += kThreadsD) {
+    conceal_columns(ent, n, a.luma + f * F, a.out_w, c0);
+    conceal_columns(ent, n, a.chroma + f * F, a.out_w, c0);
   }
 }
 
@@ -493,7 +548,7 @@ __global__ void __launch_bounds__(kThreadsScan) dropout_scan_kernel(const __grid
   if (n <= 0) return;  // whole CTA
   conceal_entries<kThreadsScan>(a, f, n, ent);
   uint16_t* plane = a.luma + (size_t)f * a.out_h * a.out_w;
-  for (int c = tid; c < a.out_w; c += kThreadsScan) conceal_column(ent, n, plane, a.out_w, c);
+  for (int c0 = tid & ~31; c0 < a.out_w; c0 += kThreadsScan) conceal_columns(ent, n, plane, a.out_w, c0);
 }
 
 // Chroma concealment of fields [f0, f0 + nf) from the entries the scan kernel
@@ -510,9 +565,9 @@ __global__ void __launch_bounds__(kConcealThreads) conceal_chroma_kernel(const _
   const int n = min(max(a.do_count[f], 0), kMaxDropouts);
   if (n == 0) return;  // whole CTA
   conceal_entries<kConcealThreads>(a, f, n, ent);
-  const int c = blockIdx.y * kConcealThreads + threadIdx.x;
+  const int c0 = blockIdx.y * kConcealThreads + (threadIdx.x & ~31);
   uint16_t* plane = a.chroma + (size_t)f * a.out_h * a.out_w;
-  if (c < a.out_w) conceal_column(ent, n, plane, a.out_w, c);
+  if (c0 < a.out_w) conceal_columns(ent, n, plane, a.out_w, c0);
 }
 
 }  // namespace
