@@ -204,9 +204,7 @@ __device__ __forceinline__ void dft16_half(float2* v) {
 
 template <int THREADS>
 __device__ __forceinline__ void fft_sync() {
-  if constexpr (THREADS == 32) {
-    __syncwarp();
-  } else if constexpr (THREADS == 64) {
+  if constexpr (THREADS == 64) {
     // two-warp transforms: threads [64 g, 64 g + 64) share barrier 1 + g.
     // Immediate barrier ids: with a register id the compiler reserves all 16
     // barriers per CTA, which caps residency at 4 CTAs per SM.
@@ -256,10 +254,10 @@ __device__ __forceinline__ void fft_pass(float2* s, const float2* __restrict__ t
 }
 
 // Full N-point transform (N a power of two, 64 <= N <= 65536), natural order
-// in and out, unnormalised.  THREADS is 32 (one warp), 64 (two warps of a
-// CTA of up to 4 such groups, synchronised on named barriers) or the CTA.
-// Caller must synchronise the transform's threads after filling s.  tid: this thread's index among the
-// transform's THREADS threads (the lane for a one-warp transform).
+// in and out, unnormalised.  THREADS is 64 (two warps of a CTA of up to 4 such
+// groups, synchronised on named barriers) or the CTA.  Caller must synchronise
+// the transform's threads after filling s.  tid: this thread's index among the
+// transform's THREADS threads.
 template <int N, int THREADS, bool INV, int NS = 1>
 __device__ __forceinline__ void smem_fft(float2* s, const float2* __restrict__ tw, int tid) {
   if constexpr (NS * 16 <= N) {
