@@ -90,8 +90,10 @@ struct cuvhs_adjoint {
     cuvhs::launch_adj_filter({th[0], th[1], th[2], th[3], d_z1, d_s, d_gv, derivs ? d_dg : nullptr}, c().stream);
   }
 
-  // The parameter-free tables of the filter (once per model).
-  void upload_filter_tables() {
+  // The parameter-free tables of the filter (once per model), on the context's
+  // stream: it does not wait for the default stream, where a copy of pageable
+  // memory may return before the data have reached the device.
+  bool upload_filter_tables() {
     const double fs = c().fmt.fs_hz;
     std::vector<double2> z(kN);
     std::vector<double> s(kN);
@@ -101,8 +103,9 @@ struct cuvhs_adjoint {
       z[k] = make_double2(z1.real(), z1.imag());
       s[k] = super_gauss(std::fabs((double)kk) * fs / (double)kN, 3.0e6, 9);
     }
-    cudaMemcpy(d_z1, z.data(), sizeof(double2) * kN, cudaMemcpyHostToDevice);
-    cudaMemcpy(d_s, s.data(), sizeof(double) * kN, cudaMemcpyHostToDevice);
+    cudaMemcpyAsync(d_z1, z.data(), sizeof(double2) * kN, cudaMemcpyHostToDevice, c().stream);
+    cudaMemcpyAsync(d_s, s.data(), sizeof(double) * kN, cudaMemcpyHostToDevice, c().stream);
+    return finish("filter tables");
   }
 
   void upload_params(const cuvhs_adjoint_params* p, bool derivs) {
@@ -267,7 +270,11 @@ cuvhs_status cuvhs_adjoint_create(const cuvhs_config* cfg, const uint8_t* sample
     a->nominal[3] = b2 / b0;
   }
   // one pass at the nominal parameters leaves the ACC gains for inspection
-  a->upload_filter_tables();
+  if (!a->upload_filter_tables()) {
+    fprintf(stderr, "cuvhs_adjoint_create: %s\n", a->err.c_str());
+    delete a;
+    return CUVHS_ERR_CUDA;
+  }
   a->build_filter(a->nominal, false);
   cudaMemsetAsync(a->d_tgt_c, 0, sizeof(float) * P * H * W, st);
   cuvhs::launch_adj_video(g, st);
