@@ -84,21 +84,6 @@ __device__ __forceinline__ float2 phase_angle2(float2 a, float2 b) {
   return make_float2(angle_octant(r.x, a), angle_octant(r.y, b));
 }
 
-// Square roots of two powers, correctly rounded for the finite normal values
-// a power takes (0 stays 0): the reciprocal square root estimate, one Newton
-// step, and a correction by the exact residual (P. Markstein, IBM J. Res.
-// Dev. 34, 1990).  Without the branch that a general square root takes for
-// subnormal values, which kept the work of successive samples apart.
-__device__ __forceinline__ float2 root2(float a, float b) {
-  float ya, yb;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(a));
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
-  const F2 x = f2(a, b), y = f2(ya, yb), g = x * y;
-  const float2 gp = parts(g);
-  const float2 s = parts(f2_fma(f2_fma(f2(-gp.x, -gp.y), g, x), y * f2(0.5f, 0.5f), g));
-  return make_float2(fmaxf(s.x, 0.0f), fmaxf(s.y, 0.0f));
-}
-
 // Predicated accesses: two words to global memory, a complex value from shared
 // memory.  (Written as an if, each became a branch of its own.)
 __device__ __forceinline__ void st_global_if(bool on, float* p, float x, float* q, float y) {
@@ -162,7 +147,8 @@ __device__ __forceinline__ void k1a_emit(const DemodArgs& a, const float2 (&z)[1
     if (r.x > a.wrap) r.x -= 6.28318530717959f;
     if (r.y > a.wrap) r.y -= 6.28318530717959f;
     const float2 hz = parts(f2_fma(f2(r), f2(a.demod_scale, a.demod_scale), f2(a.demod_offset, a.demod_offset)));
-    const float2 m = root2(power(z[qa]), power(z[qb]));
+    // (CUDA's square root, correctly rounded for every power; 2 us of the kernel's 133)
+    const float2 m = make_float2(sqrtf(power(z[qa])), sqrtf(power(z[qb])));
     e[qa] = m.x;
     e[qb] = m.y;
     st_global_if((unsigned)(i0 + T * qa) < (unsigned)nout, dem_out + T * qa, hz.x, env_out + T * qa, m.x);
