@@ -68,7 +68,12 @@ struct Design {
   int a_neg = 0, a_pos = 0, a_out = 0;
   std::vector<float2> ga;       // block spectrum of the truncated analytic kernel / kNa
   double a_tail = 0;            // relative l2 energy outside the kept support
-  float rot_re = 1, rot_im = 0;  // e^{-i d0}: nominal carrier phase step removed before atan2
+  // e^{-i d0} * 2^kRotScale: nominal carrier phase step removed before atan2.
+  // The exact factor leaves the angle as it is and keeps the rotated step out
+  // of the subnormal range, down to the smallest product of two samples: the
+  // angle's reciprocal flushes subnormal values to 0.
+  static constexpr int kRotScale = 32;
+  float rot_re = 1, rot_im = 0;
   double d0 = 0;                 // nominal phase step (rad/sample) at ire0
   float wrap = 0;                // largest FP32 step r with r + d0 (FP32) at most pi: above it the step wraps
   float demod_scale = 0;         // fs / 2pi

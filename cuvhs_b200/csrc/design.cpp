@@ -289,8 +289,8 @@ void Design::build(const Format& fmt) {
       while (wraps(wrap)) wrap = std::nextafterf(wrap, -4.0f);
       while (!wraps(std::nextafterf(wrap, 4.0f))) wrap = std::nextafterf(wrap, 4.0f);
     }
-    rot_re = (float)std::cos((double)d0f);
-    rot_im = (float)-std::sin((double)d0f);
+    rot_re = std::ldexp((float)std::cos((double)d0f), kRotScale);
+    rot_im = std::ldexp((float)-std::sin((double)d0f), kRotScale);
     demod_offset = (float)((double)d0f * (fs / (2.0 * kPi)) - fmt.ire0);
   }
 

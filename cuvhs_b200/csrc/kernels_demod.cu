@@ -60,7 +60,8 @@ __device__ __forceinline__ float angle_ratio(float2 c) {
   const float ax = fabsf(c.x), ay = fabsf(c.y);
   float inv;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(fmaxf(ax, ay)));
-  // 0/0 gives NaN, which fmaxf turns into the angle 0
+  // 0/0 gives NaN, which fmaxf turns into the angle 0; no other divisor is
+  // subnormal (the rotation scales the step up)
   return fmaxf(fminf(ax, ay) * inv, 0.0f);
 }
 __device__ __forceinline__ float angle_octant(float r, float2 c) {
@@ -130,7 +131,7 @@ __device__ __forceinline__ void k1a_emit(const DemodArgs& a, const float2 (&z)[1
   float e[16];
   const int first = lane == 0;
   const uint32_t prev = (uint32_t)__cvta_generic_to_shared(warp_last[warp]);
-  // the step of slot q: z * conj(zp) rotated by the nominal step, so the angle is small
+  // the step of slot q: z * conj(zp) rotated by the nominal step, so the angle is small (and scaled up)
   auto step = [&](int q) {
     float2 zp;
     zp.x = __shfl_up_sync(0xffffffffu, z[q].x, 1);
