@@ -424,12 +424,6 @@ bool Context::init(const cuvhs_config& c) {
   *hp_lls_fresh = LineLocState();
   hp_trial[0] = 0;
   hp_trial[1] = 1;
-  if (cudaMemcpy(d_trial, hp_trial, 2 * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
-    err = "trial track upload failed";
-    status = CUVHS_ERR_CUDA;
-    release();
-    return false;
-  }
   bool ev_ok = cudaEventCreateWithFlags(&ev_host, cudaEventDisableTiming) == cudaSuccess &&
                cudaEventCreateWithFlags(&ev_luma, cudaEventDisableTiming) == cudaSuccess &&
                cudaEventCreateWithFlags(&ev_edges, cudaEventDisableTiming) == cudaSuccess &&
@@ -451,6 +445,7 @@ bool Context::init(const cuvhs_config& c) {
     status = CUVHS_ERR_CUDA;
     return false;
   }
+  cudaMemcpyAsync(d_trial, hp_trial, 2 * sizeof(int), cudaMemcpyHostToDevice, stream);
   upload(d_ga, des.ga, stream);
   upload(d_gb, des.gb, stream);
   upload(d_gc, des.gc, stream);
@@ -463,10 +458,7 @@ bool Context::init(const cuvhs_config& c) {
                   stream);
   upload(d_hs64, des.hs64, stream);
   cudaMemsetAsync(d_guard_count, 0, sizeof(int), stream);
-  {
-    const LineLocState fresh;
-    cudaMemcpy(d_lls, &fresh, sizeof(fresh), cudaMemcpyHostToDevice);
-  }
+  cudaMemcpyAsync(d_lls, hp_lls_fresh, sizeof(LineLocState), cudaMemcpyHostToDevice, stream);
   std::vector<double> col_frac(fmt.output_line_len);
   for (int c = 0; c < fmt.output_line_len; c++) col_frac[c] = (double)c / (double)fmt.output_line_len;
   upload(d_col_frac, col_frac, stream);
@@ -831,8 +823,10 @@ bool Context::read_lls(LineLocState& st) {
 
 bool Context::write_lls(const LineLocState& st) {
   lls_reset = false;
-  if (cudaStreamSynchronize(stream) != cudaSuccess || cudaStreamSynchronize(lstream) != cudaSuccess ||
-      cudaMemcpy(d_lls, &st, sizeof(LineLocState), cudaMemcpyHostToDevice) != cudaSuccess)
+  // on the line stream, whose work reads the state next (it does not wait for the default stream)
+  if (cudaStreamSynchronize(stream) != cudaSuccess ||
+      cudaMemcpyAsync(d_lls, &st, sizeof(LineLocState), cudaMemcpyHostToDevice, lstream) != cudaSuccess ||
+      cudaStreamSynchronize(lstream) != cudaSuccess)
     return check_cuda("line-location state");
   return true;
 }

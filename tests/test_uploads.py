@@ -13,7 +13,7 @@ import cuvhs_b200 as cv
 CSRC = os.path.join(os.path.dirname(cv.__file__), "csrc")
 
 
-@pytest.mark.parametrize("source", ["adjoint_host.cpp"])
+@pytest.mark.parametrize("source", sorted(f for f in os.listdir(CSRC) if f.endswith((".cpp", ".cu"))))
 def test_no_upload_on_the_default_stream(source):
     with open(os.path.join(CSRC, source)) as f:
         copies = re.findall(r"cudaMemcpy\s*\(.*?;", f.read(), re.S)
