@@ -144,7 +144,7 @@ void Context::release() {
   hstream = nullptr;
   if (pstream) cudaStreamDestroy(pstream);
   pstream = nullptr;
-  for (cudaEvent_t* e : {&ev_ll, &ev_win, &ev_winhost, &ev_k1b, &ev_pre, &ev_guard, &ev_hs, &ev_trial, &ev_trialh, &ev_cpass}) {
+  for (cudaEvent_t* e : {&ev_ll, &ev_win, &ev_winhost, &ev_k1b, &ev_pre, &ev_guard, &ev_hs, &ev_trial, &ev_trialh, &ev_cpass, &ev_conceal}) {
     if (*e) cudaEventDestroy(*e);
     *e = nullptr;
   }
@@ -436,6 +436,7 @@ bool Context::init(const cuvhs_config& c) {
                cudaEventCreateWithFlags(&ev_trial, cudaEventDisableTiming) == cudaSuccess &&
                cudaEventCreateWithFlags(&ev_trialh, cudaEventDisableTiming) == cudaSuccess &&
                cudaEventCreateWithFlags(&ev_cpass, cudaEventDisableTiming) == cudaSuccess &&
+               cudaEventCreateWithFlags(&ev_conceal, cudaEventDisableTiming) == cudaSuccess &&
                cudaEventCreateWithFlags(&ev_guard, cudaEventDisableTiming) == cudaSuccess;
   for (cudaEvent_t* e : {&ev_prefetch, &ev_small, &ev_chroma, &ev_out_done[0], &ev_out_done[1]})
     ev_ok = ev_ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
@@ -854,6 +855,7 @@ bool Context::chroma_fields(ChromaArgs& ca, int P, const DropoutArgs* conceal, u
       begin_stage(kStageDropouts, ev_);
       launch_dropout_conceal_chroma(*conceal, f0, nf, stream);
       end_stage(kStageDropouts, ev_);
+      cudaEventRecord(ev_conceal, stream);
     }
     if (dst_chroma) {
       cudaEventRecord(ev_chroma, stream);
@@ -1010,6 +1012,9 @@ bool Context::chroma_fields(ChromaArgs& ca, int P, const DropoutArgs* conceal, u
     }
   }
   for (int f = 0; f < P; f++) hp_track[f] = computed_track[f] = plane[f];
+  // the first pass's concealment, behind luma and the dropout lists on the
+  // decode stream, may not have reached these fields yet
+  if (!again.empty() && conceal && cs != stream) cudaStreamWaitEvent(cs, ev_conceal, 0);
   for (const auto& m : again) {
     cudaMemcpyAsync(d_track + m.first, hp_track + m.first, m.second * sizeof(int), cudaMemcpyHostToDevice, cs);
     chroma_pass(m.first, m.second, true, false);

@@ -166,6 +166,7 @@ struct Context {
   // pick in hp_burst / hp_pick.
   cudaEvent_t ev_hs = nullptr, ev_trial = nullptr, ev_trialh = nullptr;  // ev_trialh: the copies to the host
   cudaEvent_t ev_cpass = nullptr;  // a chroma pass on its stream, before its concealment
+  cudaEvent_t ev_conceal = nullptr;  // a chroma pass's concealment on the decode stream
   int* d_trial = nullptr;        // {0, 1}: the trial tracks
   float* d_burst_trial = nullptr;  // [2][out_h * burst_len]
   int* d_pick = nullptr;
