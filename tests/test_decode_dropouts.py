@@ -28,7 +28,7 @@ def capture(system, mhz, fields, swap_at, per_line, longest, seed):
     line = starts[1] - starts[0]
     for f in range(1, fields):
         rows = np.arange(int(f * per_field) + 25, int((f + 1) * per_field) - 10)
-        for r in rng.choice(rows, int(per_line * rows.size)):
+        for r in rng.choice(rows, int(per_line * rows.size), replace=per_line > 1):
             s = int(starts[r] + rng.uniform(0.2, 0.9) * line)
             n = rng.integers(20, longest)
             weak[s:s + (n if n > line else min(n, int(starts[r] + 0.97 * line) - s))] = True
@@ -62,6 +62,11 @@ def unconcealed(mhz, system, x, fields):
     ("NTSC", 28.0, 20, 4, 0.6, 400),
     ("NTSC", 28.0, 20, 7, 0.4, 900),
     ("PAL", 40.0, 18, 3, 0.5, 500),
+    # runs over many lines, which overlap and come in hundreds
+    ("NTSC", 28.0, 6, 0, 0.9, 12000),
+    ("NTSC", 35.8, 6, 0, 2.0, 250),
+    ("PAL", 40.0, 6, 0, 0.9, 16000),
+    ("PAL", 28.0, 6, 0, 2.0, 200),
 ])
 def test_decode_conceals_as_the_reference_steps(monkeypatch, system, mhz, fields, swap_at, per_line, longest):
     x = capture(system, mhz, fields, swap_at, per_line, longest, 700 + swap_at)
