@@ -668,12 +668,14 @@ void edges_bits_launch(const S& e, int portions, long long max_total, cudaStream
   const int nblk = (int)((max_total + bit_edge_seg<WPT>() - 1) / bit_edge_seg<WPT>());
   const dim3 grid(nblk, 1, portions);
   launch_chained(edge_bits_count_kernel<WPT, S>, grid, dim3(kEdgeThreads), 0, st, e);
-  if (nblk <= kDirectBlocks) {
-    launch_chained(edge_bits_write_kernel<WPT, true, S>, grid, dim3(kEdgeThreads), 0, st, e);
-  } else {
-    launch_chained(edge_bits_scan_kernel<WPT, S>, dim3(1, 1, portions), dim3(kScanThreads), 0, st, e);
-    launch_chained(edge_bits_write_kernel<WPT, false, S>, grid, dim3(kEdgeThreads), 0, st, e);
+  if constexpr (WPT > 1) {  // one word a thread: always few CTAs
+    if (nblk > kDirectBlocks) {
+      launch_chained(edge_bits_scan_kernel<WPT, S>, dim3(1, 1, portions), dim3(kScanThreads), 0, st, e);
+      launch_chained(edge_bits_write_kernel<WPT, false, S>, grid, dim3(kEdgeThreads), 0, st, e);
+      return;
+    }
   }
+  launch_chained(edge_bits_write_kernel<WPT, true, S>, grid, dim3(kEdgeThreads), 0, st, e);
 }
 template <class S>
 int edges_bits_any(const S& e, int portions, long long max_total, cudaStream_t st) {
