@@ -224,11 +224,12 @@ __device__ __forceinline__ ChromaSample chroma_sample(const AdjArgs& a, int gl, 
 constexpr int kPairThreads = 64;
 constexpr int kPairs = 2;
 constexpr int kPerThread = kLineFFT / kPairThreads;  // columns a thread
+static_assert(kPairThreads == 64 && kPairs <= 4, "groups of smem_fft, a barrier each");
 
 // 1024-point band-pass of the two lines held in sm (real and imaginary parts).
 __device__ __forceinline__ void line_bandpass(float2* sm, const AdjArgs& a, int tid) {
   fft_sync<kPairThreads>();
-  smem_fft<kLineFFT, kPairThreads, false>(sm, a.tw_l, tid);
+  smem_fft<kLineFFT, false>(sm, a.tw_l, tid);
   const int lo = a.fsc_bin - a.bw_bins, hi = a.fsc_bin + a.bw_bins;
   const float scale = 1.0f / (float)kLineFFT;
   for (int k = tid; k < kLineFFT; k += kPairThreads) {
@@ -238,7 +239,7 @@ __device__ __forceinline__ void line_bandpass(float2* sm, const AdjArgs& a, int 
     sm[pidx(k)] = make_float2(x.x * m, x.y * m);
   }
   fft_sync<kPairThreads>();
-  smem_fft<kLineFFT, kPairThreads, true>(sm, a.tw_l_inv, opaque_index(tid));
+  smem_fft<kLineFFT, true>(sm, a.tw_l_inv, opaque_index(tid));
 }
 
 // Sums of K values over a pair's threads, the same in every thread: each

@@ -1,4 +1,5 @@
-// Shared-memory FP32 complex FFT for one CTA (sm_100a).
+// FP32 complex FFT parts (sm_100a): the butterflies and twiddles that every
+// transform here is made of, and a transform in shared memory by two warps.
 //
 // Stockham auto-sort, radix-16 passes (plus one radix-2/4/8 pass for sizes that
 // are not a power of 16).  Each thread holds its butterflies' inputs in
@@ -202,12 +203,16 @@ __device__ __forceinline__ void dft16_half(float2* v) {
   dft16_second<INV>(v);
 }
 
+// Barrier of a transform's THREADS threads: a CTA, or one of the groups of 64 in
+// a CTA, threads [64 g, 64 g + 64) on barrier 1 + g.
 template <int THREADS>
 __device__ __forceinline__ void fft_sync() {
   if constexpr (THREADS == 64) {
-    // two-warp transforms: threads [64 g, 64 g + 64) share barrier 1 + g.
     // Immediate barrier ids: with a register id the compiler reserves all 16
-    // barriers per CTA, which caps residency at 4 CTAs per SM.
+    // barriers per CTA, which caps residency at 4 CTAs per SM.  The CTAs here
+    // have two groups; a choice between two ids alone, as a branch or by
+    // predicates, compiled to slower line kernels (40 fields and the trials
+    // together 78 us: 79 and 83).
     const int g = threadIdx.x >> 6;
     if (g == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
     else if (g == 1) asm volatile("bar.sync 2, 64;" ::: "memory");
@@ -218,55 +223,47 @@ __device__ __forceinline__ void fft_sync() {
   }
 }
 
-// One Stockham pass of radix R on an N-point padded buffer, current span NS.
-template <int N, int THREADS, int R, int NS, bool INV>
+// One Stockham pass of radix R on an N-point padded buffer, current span NS, by
+// a group of 64 threads.
+template <int N, int R, int NS, bool INV>
 __device__ __forceinline__ void fft_pass(float2* s, const float2* __restrict__ tw, int tid) {
   constexpr int NB = N / R;
-  constexpr int PER = (NB + THREADS - 1) / THREADS;
+  constexpr int PER = NB / 64;
+  static_assert(NB % 64 == 0, "whole butterflies a thread");
   float2 v[PER][R];
 #pragma unroll
   for (int p = 0; p < PER; p++) {
-    const int j = tid + p * THREADS;
-    if ((NB % THREADS) == 0 || j < NB) {
+    const int j = tid + p * 64;
 #pragma unroll
-      for (int r = 0; r < R; r++) v[p][r] = s[pidx(j + r * NB)];
-      if constexpr (NS > 1) {
-        const int k = j & (NS - 1);
-        const float2* twp = tw + (NS - 16) + k;
+    for (int r = 0; r < R; r++) v[p][r] = s[pidx(j + r * NB)];
+    if constexpr (NS > 1) {
+      const int k = j & (NS - 1);
+      const float2* twp = tw + (NS - 16) + k;
 #pragma unroll
-        for (int r = 1; r < R; r++) v[p][r] = cmul_tw<INV>(v[p][r], __ldg(&twp[(r - 1) * NS]));
-      }
-      dft<R, INV>(v[p]);
+      for (int r = 1; r < R; r++) v[p][r] = cmul_tw<INV>(v[p][r], __ldg(&twp[(r - 1) * NS]));
     }
+    dft<R, INV>(v[p]);
   }
-  fft_sync<THREADS>();
+  fft_sync<64>();
 #pragma unroll
   for (int p = 0; p < PER; p++) {
-    const int j = tid + p * THREADS;
-    if ((NB % THREADS) == 0 || j < NB) {
-      const int k = j & (NS - 1);
-      const int base = (j / NS) * NS * R + k;
+    const int j = tid + p * 64;
+    const int k = j & (NS - 1);
+    const int base = (j / NS) * NS * R + k;
 #pragma unroll
-      for (int r = 0; r < R; r++) s[pidx(base + r * NS)] = v[p][dft_slot<R>(r)];
-    }
+    for (int r = 0; r < R; r++) s[pidx(base + r * NS)] = v[p][dft_slot<R>(r)];
   }
-  fft_sync<THREADS>();
+  fft_sync<64>();
 }
 
-// Full N-point transform (N a power of two, 64 <= N <= 65536), natural order
-// in and out, unnormalised.  THREADS is 64 (two warps of a CTA of up to 4 such
-// groups, synchronised on named barriers) or the CTA.  Caller must synchronise
-// the transform's threads after filling s.  tid: this thread's index among the
-// transform's THREADS threads.
-template <int N, int THREADS, bool INV, int NS = 1>
+// Full N-point transform by a group of 64 threads (N a power of two, at least
+// 1024), natural order in and out, unnormalised.  The caller synchronises the
+// group after filling s.  tid: this thread's index in its group.
+template <int N, bool INV, int NS = 1>
 __device__ __forceinline__ void smem_fft(float2* s, const float2* __restrict__ tw, int tid) {
-  if constexpr (NS * 16 <= N) {
-    fft_pass<N, THREADS, 16, NS, INV>(s, tw, tid);
-    smem_fft<N, THREADS, INV, NS * 16>(s, tw, tid);
-  } else if constexpr (NS < N) {
-    constexpr int R = N / NS;  // 2, 4 or 8
-    static_assert(R == 2 || R == 4 || R == 8, "N must be a power of two");
-    fft_pass<N, THREADS, R, NS, INV>(s, tw, tid);
+  if constexpr (NS < N) {
+    fft_pass<N, fft_radix(N, NS), NS, INV>(s, tw, tid);
+    smem_fft<N, INV, NS * fft_radix(N, NS)>(s, tw, tid);
   }
 }
 
