@@ -23,6 +23,8 @@ constexpr int kMaxPulses = 800;        // pulses kept per field
 constexpr int kPhaseSlots = 32;        // phase clocks recorded per field or sample (inspection)
 constexpr int kMaxDropouts = 512;      // TBC dropout entries per field
 constexpr int kMaxRfDropouts = 128;    // RF-domain dropout spans per field
+constexpr int kMaxLineLen = 1135;      // output columns a line kernel's threads cover (NTSC 910, PAL 1135)
+constexpr int kMaxFieldLines = 320;    // line starts of a field held in shared memory (NTSC 264, PAL 314)
 constexpr int kMaxBurstLen = 48;       // burst window width bound, output samples (NTSC 36, PAL 40)
 enum PulseType { kHsync = 0, kEq1 = 1, kVsync = 2, kEq2 = 3 };
 enum VideoSystem { kNtsc = 0, kPal = 1 };
@@ -112,6 +114,8 @@ struct Design {
   // build() once per sample rate per process; later calls copy the result
   // (thread-safe).  Contexts of one rate then share the FP64 design work.
   void build_cached(const Format& fmt);
+  // What the line kernels take for granted of a system and this one does not meet; null if it meets all.
+  const char* unmet_geometry(const Format& fmt) const;
 };
 
 // Half-support (samples each side) of the truncated K1a kernel at a capture

@@ -374,6 +374,19 @@ void Design::build(const Format& fmt) {
   if (bw_bins < 10) bw_bins = 10;
 }
 
+const char* Design::unmet_geometry(const Format& fmt) const {
+  const int slot = fmt.line_fft / 16;  // columns or bins of a slot of the line transform
+  if (fmt.line_fft != 1024 && fmt.line_fft != 2048) return "the line transform has 1024 or 2048 points";
+  if (fsc_bin - bw_bins <= 3 * slot || fsc_bin + bw_bins >= 5 * slot)
+    return "the chroma band lies in slots 3 and 4 of the line transform";
+  if (fmt.burst_start < 0 || fmt.burst_start + fmt.burst_len > 2 * slot)
+    return "the burst lies in the first two slots of the line transform";
+  if (fmt.burst_len != 36 && fmt.burst_len != 40) return "the burst window has 36 or 40 samples";
+  if (fmt.output_line_len > kMaxLineLen) return "a line has at most 1135 columns";
+  if (fmt.output_field_lines >= kMaxFieldLines) return "a field has fewer than 320 lines";
+  return nullptr;
+}
+
 }  // namespace cuvhs
 
 namespace cuvhs {

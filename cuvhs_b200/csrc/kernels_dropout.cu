@@ -95,7 +95,6 @@ __device__ __forceinline__ int block_excl_sum(int v, int* wsh, int* total) {
   return res;
 }
 
-constexpr int kMaxFieldLines = 320;  // line starts held in shared memory: 264 NTSC, 314 PAL
 struct MapScratch {
   double ll[kMaxFieldLines];  // the field's line starts from the first active line
   int rf_s[kMaxRfDropouts], rf_e[kMaxRfDropouts];

@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(32 * kHsyncWarps) hsync_kernel(const __grid_co
 // address a thread, one range test a pixel and no conversions that a bit
 // pattern replaces.
 constexpr int kLumaWindowMax = 4096;
-constexpr int kLumaColumns = (1135 + kLumaThreads - 1) / kLumaThreads;  // pixels a thread, the widest line (PAL)
+constexpr int kLumaColumns = (kMaxLineLen + kLumaThreads - 1) / kLumaThreads;  // pixels a thread, the widest line
 // Samples staged per row: a line and 6%, with room for the taps.
 inline int luma_window(double one_us) {
   return std::min(kLumaWindowMax, ((int)(one_us * 64.0 * 1.06) + 32 + 31) & ~31);

@@ -375,6 +375,11 @@ bool Context::init(const cuvhs_config& c) {
   dc_correct = c.dc_correct != 0;
   fmt.init(c.sample_rate_mhz, c.system);
   des.build_cached(fmt);
+  if (const char* unmet = des.unmet_geometry(fmt)) {
+    err = std::string("unsupported system: the kernels assume that ") + unmet;
+    status = CUVHS_ERR_UNSUPPORTED;
+    return false;
+  }
   spp = fmt.spp;
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
