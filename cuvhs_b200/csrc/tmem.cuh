@@ -24,10 +24,14 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, int warp) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
 }
-// After a __syncthreads() behind every thread's last load.
+// After a __syncthreads() behind every thread's last load.  The warp frees as
+// one (.aligned), whatever branches its threads took since.
 template <int COLS>
 __device__ __forceinline__ void tmem_free(uint32_t base, int warp) {
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(COLS));
+  if (warp == 0) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(COLS));
+  }
 }
 // The address of a warp's own columns: its lanes, `cols` columns a warp.
 __device__ __forceinline__ uint32_t tmem_own(uint32_t base, int warp, int cols) {
