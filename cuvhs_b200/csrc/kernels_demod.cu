@@ -148,7 +148,8 @@ __device__ __forceinline__ void k1a_emit(const DemodArgs& a, const float2 (&z)[1
     if (r.x > a.wrap) r.x -= 6.28318530717959f;
     if (r.y > a.wrap) r.y -= 6.28318530717959f;
     const float2 hz = parts(f2_fma(f2(r), f2(a.demod_scale, a.demod_scale), f2(a.demod_offset, a.demod_offset)));
-    // (CUDA's square root, correctly rounded for every power; 2 us of the kernel's 133)
+    // (CUDA's square root, correctly rounded for every power: 2 us more than an
+    // estimate with one correction, which is not)
     const float2 m = make_float2(sqrtf(power(z[qa])), sqrtf(power(z[qb])));
     e[qa] = m.x;
     e[qb] = m.y;
@@ -182,14 +183,15 @@ __device__ __forceinline__ void k1a_emit(const DemodArgs& a, const float2 (&z)[1
 // K1a: u8 -> analytic signal -> phase step + envelope, blocks 2x and 2x+1 of
 // the tile (the second may lie past the tile's end).
 //
-// Bound by an SM's units side by side, none of them full: FP32 pipe 49%, shared
-// memory 46%, load/store 41%, issue 57% of cycles; DRAM 9%.  64 registers and
-// 51 KB of shared memory put four CTAs on an SM, in different parts of their
-// transforms (three at 80 registers: 130 us).  The second block's half
-// spectrum waits in shared memory, and U is exchanged in the transform's own
-// buffer.  40 fields at 28 MHz: 171 -> 126 us, 168 MB of interface traffic at
-// 984 -> 1,335 GB/s.  (Two pairs of blocks in the two lanes of packed
-// arithmetic, four blocks a CTA at 128 registers and two CTAs an SM: 187 us.)
+// Bound by an SM's units side by side, none of them full: FP32 pipe 49%,
+// load/store 42%, issue 62% of cycles; DRAM 11%.  64 registers (16 bytes a
+// thread spilled) and 51 KB of shared memory put four CTAs on an SM, in
+// different parts of their transforms (three at 80 registers: 3% slower).  The
+// second block's half spectrum waits in shared memory, and U is exchanged in
+// the transform's own buffer.  40 fields at 28 MHz under ncu: 172 -> 134 us, 168
+// MB of interface traffic at 978 -> 1,253 GB/s.  (Two pairs of blocks in the
+// two lanes of packed arithmetic, four blocks a CTA at 128 registers and two
+// CTAs an SM: 187 us.)
 template <int FMT, class Src>
 __global__ void __launch_bounds__(kThreadsA, 4) k1a_kernel(const __grid_constant__ Src src, int f_begin) {
   constexpr int N = Design::kNa, T = kThreadsA;
@@ -313,9 +315,9 @@ __device__ __forceinline__ void k1b_emit(const DemodArgs& a, const float2 (&z)[1
 // block's spectrum (64 KB, which shared memory does not hold twice more) waits
 // in tensor memory, each thread's 32 words in columns of its own.  Both
 // inverses in lockstep at 128 registers and one CTA an SM left every unit
-// below 38% (issue 44%); now FP32 pipe 41%, shared memory 44%, load/store 37%,
-// issue 52%, DRAM 17%.  40 fields at 28 MHz: 179 -> 140 us, 227 MB of
-// interface traffic at 1,266 -> 1,618 GB/s.
+// below 38% (issue 44%); now FP32 pipe 40%, load/store 36%, issue 51%, DRAM 15%
+// (36 bytes a thread spilled).  40 fields at 28 MHz under ncu: 179 -> 149 us,
+// 227 MB of interface traffic at 1,263 -> 1,517 GB/s.
 template <class Src>
 __global__ void __launch_bounds__(kThreadsB, 2) k1b_kernel(const __grid_constant__ Src src, int f_begin) {
   constexpr int N = Design::kNb, T = kThreadsB;

@@ -3,11 +3,12 @@
 // A packed instruction does two FP32 operations, each rounded as the scalar
 // one, in one issue slot (the FP32 pipe takes two cycles for it: 125 lane
 // operations a clock and SM measured, against 110 for scalar instructions).
-// The FFT kernels are bound by instruction issue (54-71% of cycles issue
-// while the FP32 pipe is 30-37% busy), so halving the instructions of the same
-// arithmetic is worth what fewer operations would be.  Operands may name
-// either half of a register pair for each lane, with a sign: broadcasting,
-// swapping and negating the parts of a complex value cost no instruction.
+// In scalar arithmetic the FFT kernels were bound by instruction issue (54-71%
+// of cycles issued while the FP32 pipe was 30-37% busy), so halving the
+// instructions of the same arithmetic is worth what fewer operations would be.
+// Operands may name either half of a register pair for each lane, with a sign:
+// broadcasting, swapping and negating the parts of a complex value cost no
+// instruction.
 #pragma once
 #include <cuda_runtime.h>
 
